@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "lb_ff.cuh"
+
 namespace lb {
 
 // ---------------------------------------------------------------- D3Q19 table
@@ -328,36 +330,57 @@ __device__ __forceinline__ void d3q19_sc_sum_native(const float (&ps)[19], float
                           ((ps[10] + ps[14]) + (ps[16] + ps[18]))));
 }
 
+// A Zou-He line of the reference, (float)((double)g + c (double)ru - 0.5
+// (double)t) with its double literals: in pairs of floats, or as written where
+// these do not decide the rounding (lb_ff.cuh)
+__device__ __forceinline__ float zou_he_face(float g, double c, float ru, float t) {
+    float v;
+    if (ff_face(g, ff_const(c), ru, t, v)) return v;
+    return (float)((double)g + c * (double)ru - 0.5 * (double)t);
+}
+// the density of a velocity inlet, inv = 1 / (1 - ux_in) as two floats
+__device__ __forceinline__ float zou_he_rho(float a, float b, float ux_in, FF inv) {
+    float v;
+    if (ff_ratio(a, b, inv, 0.f, v)) return v;
+    return (float)(((double)a + 2. * (double)b) / (1. - (double)ux_in));
+}
+// the velocity of a pressure outlet, inv = 1 / rho_out as two floats
+__device__ __forceinline__ float zou_he_u(float a, float b, float rho_out, FF inv) {
+    float v;
+    if (ff_ratio(a, b, inv, -1.f, v)) return v;
+    return (float)(-1. + ((double)a + 2. * (double)b) / (double)rho_out);
+}
+
 // Zou-He velocity inlet at the west face, reference src/collision.cu:412-430
 // (the reference's double literals promote these lines to FP64)
-__device__ __forceinline__ void d3q19_zou_he_west(float (&g)[19], float ux_in) {
+__device__ __forceinline__ void d3q19_zou_he_west(float (&g)[19], float ux_in, FF inv) {
     const float a = g[0] + g[3] + g[4] + g[5] + g[6] + g[15] + g[16] + g[17] + g[18];
     const float b = g[2] + g[11] + g[12] + g[13] + g[14];
-    const float rho = (float)(((double)a + 2. * (double)b) / (1. - (double)ux_in));
+    const float rho = zou_he_rho(a, b, ux_in, inv);
     const float ru = rho * ux_in;
     const float ty = g[3] + g[15] + g[16] - g[4] - g[17] - g[18];
     const float tz = g[5] + g[11] + g[15] - g[6] - g[16] - g[18];
-    g[1]  = (float)((double)g[2]  + (1. / 3.) * (double)ru);
-    g[8]  = (float)((double)g[11] + (1. / 6.) * (double)ru + 0.5 * (double)ty);
-    g[7]  = (float)((double)g[12] + (1. / 6.) * (double)ru - 0.5 * (double)ty);
-    g[9]  = (float)((double)g[14] + (1. / 6.) * (double)ru - 0.5 * (double)tz);
-    g[10] = (float)((double)g[13] + (1. / 6.) * (double)ru + 0.5 * (double)tz);
+    g[1]  = zou_he_face(g[2], 1. / 3., ru, 0.f);
+    g[8]  = zou_he_face(g[11], 1. / 6., ru, -ty);
+    g[7]  = zou_he_face(g[12], 1. / 6., ru, ty);
+    g[9]  = zou_he_face(g[14], 1. / 6., ru, tz);
+    g[10] = zou_he_face(g[13], 1. / 6., ru, -tz);
 }
 
 // Zou-He pressure outlet at the east face, reference src/collision.cu:432-451;
 // the last two lines read the f11 written just before, as the reference does
-__device__ __forceinline__ void d3q19_zou_he_east(float (&g)[19], float rho_out) {
+__device__ __forceinline__ void d3q19_zou_he_east(float (&g)[19], float rho_out, FF inv) {
     const float a = g[0] + g[3] + g[4] + g[5] + g[6] + g[15] + g[16] + g[17] + g[18];
     const float b = g[1] + g[7] + g[8] + g[9] + g[10];
-    const float ux = (float)(-1. + ((double)a + 2. * (double)b) / (double)rho_out);
+    const float ux = zou_he_u(a, b, rho_out, inv);
     const float ru = rho_out * ux;
     const float ty = g[3] + g[15] + g[16] - g[4] - g[17] - g[18];
-    g[2]  = (float)((double)g[1] - (1. / 3.) * (double)ru);
-    g[11] = (float)((double)g[8] - (1. / 6.) * (double)ru - 0.5 * (double)ty);
-    g[12] = (float)((double)g[7] - (1. / 6.) * (double)ru + 0.5 * (double)ty);
+    g[2]  = zou_he_face(g[1], 1. / 3., -ru, 0.f);
+    g[11] = zou_he_face(g[8], 1. / 6., -ru, ty);
+    g[12] = zou_he_face(g[7], 1. / 6., -ru, -ty);
     const float tz = g[5] + g[11] + g[15] - g[6] - g[16] - g[18];
-    g[14] = (float)((double)g[9]  - (1. / 6.) * (double)ru + 0.5 * (double)tz);
-    g[13] = (float)((double)g[10] - (1. / 6.) * (double)ru - 0.5 * (double)tz);
+    g[14] = zou_he_face(g[9], 1. / 6., -ru, -tz);
+    g[13] = zou_he_face(g[10], 1. / 6., -ru, tz);
 }
 
 // ---------------------------------------------------------------- BGK, D2Q9
@@ -459,21 +482,19 @@ __device__ __forceinline__ void d2q9_collide_native(float (&g)[9], float Fx, flo
 }
 
 // Zou-He west inlet / east outlet, reference src/collision.cu:210-262
-__device__ __forceinline__ void d2q9_zou_he_west(float (&g)[9], float ux_in) {
-    const float a = g[0] + g[2] + g[4], b = g[3] + g[7] + g[6];
-    const float r = (float)(((double)a + 2. * (double)b) / (1. - (double)ux_in));
+__device__ __forceinline__ void d2q9_zou_he_west(float (&g)[9], float ux_in, FF inv) {
+    const float r = zou_he_rho(g[0] + g[2] + g[4], g[3] + g[7] + g[6], ux_in, inv);
     const float ru = r * ux_in;
-    g[1] = (float)((double)g[3] + (2. / 3.) * (double)ru);
-    g[5] = (float)((double)g[7] + (1. / 6.) * (double)ru - 0.5 * (double)(g[2] - g[4]));
-    g[8] = (float)((double)g[6] + (1. / 6.) * (double)ru - 0.5 * (double)(g[4] - g[2]));
+    g[1] = zou_he_face(g[3], 2. / 3., ru, 0.f);
+    g[5] = zou_he_face(g[7], 1. / 6., ru, g[2] - g[4]);
+    g[8] = zou_he_face(g[6], 1. / 6., ru, g[4] - g[2]);
 }
-__device__ __forceinline__ void d2q9_zou_he_east(float (&g)[9], float rho_out) {
-    const float a = g[0] + g[2] + g[4], b = g[1] + g[5] + g[8];
-    const float vx = (float)(-1. + ((double)a + 2. * (double)b) / (double)rho_out);
+__device__ __forceinline__ void d2q9_zou_he_east(float (&g)[9], float rho_out, FF inv) {
+    const float vx = zou_he_u(g[0] + g[2] + g[4], g[1] + g[5] + g[8], rho_out, inv);
     const float ru = rho_out * vx;
-    g[3] = (float)((double)g[1] - (2. / 3.) * (double)ru);
-    g[7] = (float)((double)g[5] - (1. / 6.) * (double)ru + 0.5 * (double)(g[2] - g[4]));
-    g[6] = (float)((double)g[8] - (1. / 6.) * (double)ru + 0.5 * (double)(g[4] - g[2]));
+    g[3] = zou_he_face(g[1], 2. / 3., -ru, 0.f);
+    g[7] = zou_he_face(g[5], 1. / 6., -ru, g[4] - g[2]);
+    g[6] = zou_he_face(g[8], 1. / 6., -ru, g[2] - g[4]);
 }
 
 // Shan-Chen interaction of the D2Q9 step, reference src/collision.cu:78-96:
@@ -528,6 +549,8 @@ __device__ __forceinline__ float lb_expf(float x) {
 
 // psi(rho) forms of the Shan-Chen pseudo-potential
 __device__ __forceinline__ float psi_ref(float rho) {  // src/collision.cu:293
+    float v;
+    if (ff_psi_ref(rho, v)) return v;  // in pairs of floats (lb_ff.cuh)
     return (float)(4. * exp(-200. / (double)rho));
 }
 __device__ __forceinline__ float psi_exp1(float rho) { return 1.f - lb_expf(-rho); }

@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(D2_BLOCK) d2q9_fused_kernel(const D2Args a) {
     }
     if (MODE == MODE_REF) {
         if (x == 0 && a.dev == 0)
-            d2q9_zou_he_west(g, a.ux_in);
+            d2q9_zou_he_west(g, a.ux_in, a.inv_in);
         else if (x == a.W - 1 && a.dev == a.ndev - 1)
-            d2q9_zou_he_east(g, a.rho_out);
+            d2q9_zou_he_east(g, a.rho_out, a.inv_out);
     }
     float rho, ux, uy;
     d2q9_moments(g, rho, ux, uy);
@@ -256,9 +256,9 @@ __global__ void __launch_bounds__(D2_BLOCK) d2q9_collide_kernel(const D2Args a) 
 #pragma unroll
     for (int k = 0; k < 9; k++) g[k] = a.dst.f[d2_opp(k)][o];
     if (x == 0 && a.dev == 0)
-        d2q9_zou_he_west(g, a.ux_in);
+        d2q9_zou_he_west(g, a.ux_in, a.inv_in);
     else if (x == a.W - 1 && a.dev == a.ndev - 1)
-        d2q9_zou_he_east(g, a.rho_out);
+        d2q9_zou_he_east(g, a.rho_out, a.inv_out);
     float rho, ux, uy;
     d2q9_moments(g, rho, ux, uy);
     float ex = ux, ey = uy;
@@ -308,7 +308,8 @@ __global__ void d2q9_equilibrium_kernel(Pop<9> p, const float *rho, const float 
 // ---------------------------------------------------------------- launchers
 static dim3 grid2(int W, int H) { return dim3((W + D2_BLOCK - 1) / D2_BLOCK, H); }
 
-cudaError_t launch_d2q9_fused(const D2Args &a, int mode, bool mom, bool plot, cudaStream_t s) {
+cudaError_t launch_d2q9_fused(const D2Args &a0, int mode, bool mom, bool plot, cudaStream_t s) {
+    const D2Args a = with_zou_he(a0);
     const dim3 g = grid2(a.W, a.H), b(D2_BLOCK);
     // the Shan-Chen pass runs for G < 0 in reference mode (src/collision.cu:352)
     // and for any G != 0 in native mode
@@ -345,7 +346,8 @@ cudaError_t launch_d2q9_fused(const D2Args &a, int mode, bool mom, bool plot, cu
     return cudaGetLastError();
 }
 
-cudaError_t launch_d2q9_fused_pdl(const D2Args &a, int mode, bool mom, cudaStream_t s) {
+cudaError_t launch_d2q9_fused_pdl(const D2Args &a0, int mode, bool mom, cudaStream_t s) {
+    const D2Args a = with_zou_he(a0);
     if (a.G != 0.f) return cudaErrorInvalidValue;  // no Shan-Chen pass here
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid2(a.W, a.H);
@@ -369,7 +371,8 @@ cudaError_t launch_d2q9_stream_swap(const Pop<9> &p, const uint8_t *sb, int W, i
     return cudaGetLastError();
 }
 
-cudaError_t launch_d2q9_collide(const D2Args &a, bool plot, cudaStream_t s) {
+cudaError_t launch_d2q9_collide(const D2Args &a0, bool plot, cudaStream_t s) {
+    const D2Args a = with_zou_he(a0);
     const dim3 g = grid2(a.W, a.H), b(D2_BLOCK);
     if (plot) d2q9_collide_kernel<true><<<g, b, 0, s>>>(a);
     else d2q9_collide_kernel<false><<<g, b, 0, s>>>(a);

@@ -96,9 +96,9 @@ __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
         for (int k = 0; k < 19; k++)
             g[k] = ld_stream(a.src.f[k] + o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k)));
         if (x == 0 && a.dev == 0)
-            d3q19_zou_he_west(g, a.ux_in);
+            d3q19_zou_he_west(g, a.ux_in, a.inv_in);
         else if (x == a.W - 1 && a.dev == a.ndev - 1)
-            d3q19_zou_he_east(g, a.rho_out);
+            d3q19_zou_he_east(g, a.rho_out, a.inv_out);
     }
     float rho, ux, uy, uz;
     if (MODE == MODE_NATIVE) StepArith<S>::moments(g, a, rho, ux, uy, uz);
@@ -201,9 +201,9 @@ __global__ void __launch_bounds__(D3_BLOCK) d3q19_collide_kernel(const D3Args a)
 #pragma unroll
     for (int k = 0; k < 19; k++) g[k] = a.dst.f[d3_opp(k)][o];
     if (x == 0 && a.dev == 0)
-        d3q19_zou_he_west(g, a.ux_in);
+        d3q19_zou_he_west(g, a.ux_in, a.inv_in);
     else if (x == a.W - 1 && a.dev == a.ndev - 1)
-        d3q19_zou_he_east(g, a.rho_out);
+        d3q19_zou_he_east(g, a.rho_out, a.inv_out);
     float rho, ux, uy, uz;
     d3q19_moments(g, rho, ux, uy, uz);
     a.ux[o] = ux; a.uy[o] = uy; a.uz[o] = uz; a.rho[o] = rho;
@@ -306,7 +306,8 @@ __global__ void from_storage_kernel(const S *src, float *dst, long n, float wr) 
 // ---------------------------------------------------------------- launchers
 static dim3 grid_of(int W, int H, int D) { return dim3((W + D3_BLOCK - 1) / D3_BLOCK, H, D); }
 
-cudaError_t launch_d3q19_fused(const D3Args &a, int mode, bool mom, bool plot, cudaStream_t s) {
+cudaError_t launch_d3q19_fused(const D3Args &a0, int mode, bool mom, bool plot, cudaStream_t s) {
+    const D3Args a = with_zou_he(a0);
     const dim3 g = grid_of(a.W, a.H, a.D), b(D3_BLOCK);
 #define LB_D3_CASE(M, MO, PL)                                                    \
     if (mode == M && mom == MO && plot == PL) {                                  \
@@ -445,7 +446,8 @@ cudaError_t launch_d3q19_stream_swap(const Pop<19> &p, const uint8_t *sb, int W,
     return cudaGetLastError();
 }
 
-cudaError_t launch_d3q19_collide(const D3Args &a, bool plot, cudaStream_t s) {
+cudaError_t launch_d3q19_collide(const D3Args &a0, bool plot, cudaStream_t s) {
+    const D3Args a = with_zou_he(a0);
     if (plot)
         d3q19_collide_kernel<true><<<grid_of(a.W, a.H, a.D), D3_BLOCK, 0, s>>>(a);
     else

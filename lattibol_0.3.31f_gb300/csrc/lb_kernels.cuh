@@ -36,6 +36,7 @@ struct D3Args {
     int z_lo, z_skip;       // planes updated: z = z_lo + blockIdx.z * (1 + z_skip) (slabs;
                             // 0, 0 = every plane, blockIdx.z itself)
     float rho_ref;          // 16-bit storage: sum_k wr[k], the density the offsets carry
+    FF inv_in, inv_out;     // reference mode: 1 / (1 - ux_in), 1 / rho_out (set by the launchers)
 };
 
 // The native step's arithmetic for storage type S: FP32 works on f itself,
@@ -84,7 +85,16 @@ struct D2Args {
     float corr[9];
     float4 *probe;          // as D3Args: (ux, uy, 0, rho) of node probe_o every step
     int probe_o;
+    FF inv_in, inv_out;     // as D3Args
 };
+
+// the arguments with the reference mode's Zou-He reciprocals
+template <typename Args> Args with_zou_he(const Args &a0) {
+    Args a = a0;
+    a.inv_in = ff_const(1. / (1. - (double)a.ux_in));
+    a.inv_out = ff_const(1. / (double)a.rho_out);
+    return a;
+}
 
 // D3Q19
 cudaError_t launch_d3q19_fused(const D3Args &a, int mode, bool mom, bool plot, cudaStream_t s);
