@@ -177,6 +177,11 @@ typedef enum {
 #define LB_TUNE_REVERSE 0x001  /* sweep the lattice in the opposite order on every
                                   other step, so a step starts where the previous
                                   one ended and its last writes are still in L2 */
+#define LB_TUNE_MARCH 0x002    /* D2Q9 native mode without Shan-Chen: one launch
+                                  advances three steps by warps that march down
+                                  strips, the time levels in between in registers
+                                  (goes before LB_TUNE_TBLOCK; part of the default
+                                  on lattices of more than 2^20 nodes) */
 #define LB_TUNE_TBLOCK 0x020   /* D2Q9 native mode without Shan-Chen: temporal
                                   blocking, one launch advances several steps of a
                                   tile and its halo in shared memory */

@@ -41,6 +41,7 @@ struct lb_ctx {
     float corr[19] = {0};
     float wr[19] = {0};                  // 16-bit storage offsets w_k * rho_ref
     int tune = 0;                        // LB_TUNE_* bits in effect
+    uint16_t *wmask = nullptr;           // marching strips: upstream-wall masks
     bool closure_on = false;             // learned closure sets the local relaxation time
     ClosureArgs closure{};
     bool flags_set = false;
@@ -92,7 +93,12 @@ int cuda_fail(lb_ctx *c, const char *where, cudaError_t e) {
 // Shan-Chen) measured 48.5 vs 24.1 GLUPS at 256^2, 11.1 vs 5.8 at 128^2 and
 // 73.3 vs 60.9 at 512^2, but 94.7 vs 101.5 at 1024^2 (a step then streams
 // from L2 faster than the blocks recompute their halos), so they are the
-// default up to TBLOCK_DEFAULT_MAX_NODES.  D3Q19 Shan-Chen without walls: the
+// default up to TBLOCK_DEFAULT_MAX_NODES.  Beyond MARCH_DEFAULT_MIN_NODES the
+// marching strips (three steps per launch) are: 1100x1000 139 vs 103 GLUPS,
+// 1568x1024 157 vs 81, 4096x2048 203 vs 82.  In between one launch per step
+// stays (900^2: 99, the strips 115; 720^2: 97 and 90): there the strips have
+// too few warps to gain much, and a 1024^2 lattice is held to one launch per
+// step by its launch count.  D3Q19 Shan-Chen without walls: the
 // staged single-pass step measured 28.6 / 34.1 / 34.2 GLUPS (FP32 / FP16 /
 // BF16) at 256^3 against 26.4 / 31.5 / 31.5 for the density pass + fused step
 // (34.9 / 40.3 / 40.4 with compact stages, two steps per loop iteration, 3
@@ -101,6 +107,7 @@ constexpr int LB_TUNE_LIBRARY_DEFAULT_D3 = LB_TUNE_REVERSE | LB_TUNE_SC_STAGED;
 constexpr int LB_TUNE_LIBRARY_DEFAULT_D2 = LB_TUNE_PDL;
 constexpr int TBLOCK_DEFAULT_SHAPE = 5;
 constexpr long TBLOCK_DEFAULT_MAX_NODES = 1L << 19;
+constexpr long MARCH_DEFAULT_MIN_NODES = 1L << 20;
 
 const double W3[3] = {1.0 / 3.0, 1.0 / 18.0, 1.0 / 36.0};
 const double W2[3] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 36.0};
@@ -168,10 +175,30 @@ int tblock_variant(const lb_ctx *c) {
     return tblock_steps(v) > 0 ? v : TBLOCK_DEFAULT_SHAPE;
 }
 
-// launches of temporal blocks per captured graph: even, so that a graph
-// returns to the set it started from
-int tblock_graph_launches(const lb_ctx *c, int steps_per_launch) {
+// the marching strips advance a launch of march_steps_per_launch() steps: D2Q9
+// native mode without Shan-Chen, and the tuning asks for them
+bool march_on(const lb_ctx *c) {
+    return c->Q == 9 && !sc_on(c) && c->cfg.mode == LB_MODE_NATIVE && (c->tune & LB_TUNE_MARCH);
+}
+
+// steps per launch of the multi-step kernel in effect (0: one launch per step)
+int multi_steps(const lb_ctx *c) {
+    if (march_on(c)) return march_steps_per_launch();
+    return tblock_steps(tblock_variant(c));
+}
+
+// multi-step launches per captured graph: even, so that a graph returns to
+// the set it started from
+int multi_graph_launches(const lb_ctx *c, int steps_per_launch) {
     return std::max(2, (c->cfg.graph_steps / steps_per_launch) & ~1);
+}
+
+// the marching strips' upstream-wall masks after the flags changed
+int update_wall_mask(lb_ctx *c, const char *where) {
+    if (!c->any_wall || !march_on(c)) return LB_OK;
+    if (!c->wmask) LB_TRY(c, where, cudaMalloc(&c->wmask, sizeof(uint16_t) * c->stride));
+    LB_TRY(c, where, launch_d2q9_wall_mask(c->flags, c->wmask, c->cfg.nx, c->cfg.ny, c->stream));
+    return LB_OK;
 }
 
 // the step kernels write the cursor probe themselves (every step path does;
@@ -307,6 +334,15 @@ cudaError_t step_once(lb_ctx *c, int from, bool moments) {
                              false, c->stream);
 }
 
+// one launch of the multi-step kernel, set `from` to set 1-from
+cudaError_t multi_once(lb_ctx *c, int from, bool moments) {
+    c->launches += 1;
+    if (march_on(c))
+        return launch_d2q9_march(d2_args(c, from), c->any_wall ? c->wmask : nullptr, moments,
+                                 c->stream);
+    return launch_d2q9_tblock(d2_args(c, from), tblock_variant(c), moments, c->stream);
+}
+
 int graph_for(lb_ctx *c, int from, cudaGraphExec_t *out) {
     if (c->graph[from]) { *out = c->graph[from]; return LB_OK; }
     cudaGraph_t graph;
@@ -315,11 +351,10 @@ int graph_for(lb_ctx *c, int from, cudaGraphExec_t *out) {
            cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int set = from;
     cudaError_t e = cudaSuccess;
-    const int tv = tblock_variant(c);
-    if (tv) {
-        const int L = tblock_graph_launches(c, tblock_steps(tv));
+    if (const int T = multi_steps(c)) {
+        const int L = multi_graph_launches(c, T);
         for (int i = 0; i < L && e == cudaSuccess; i++) {
-            e = launch_d2q9_tblock(d2_args(c, set), tv, false, c->stream);
+            e = multi_once(c, set, false);
             set = 1 - set;
         }
     } else {
@@ -432,11 +467,11 @@ int lb_create(const lb_config *cfg, lb_ctx **out) {
     if (c->cfg.graph_steps <= 0) c->cfg.graph_steps = 64;
     c->cfg.graph_steps += c->cfg.graph_steps & 1;  // even: a graph returns to its start set
     if (!(c->cfg.rho_ref > 0.f)) c->cfg.rho_ref = 1.f;
-    // explicit: the bits the header defines (REVERSE, PDL, TBLOCK, SC_STAGED,
-    // SC_NO_TMA, the block shape); any other bit is ignored
-    constexpr int kTuneBits = LB_TUNE_REVERSE | LB_TUNE_PDL | LB_TUNE_TBLOCK | LB_TUNE_SC_STAGED |
-                              LB_TUNE_SC_NO_TMA | LB_TUNE_TBLOCK_SHAPE(0x1f);
-    static_assert(kTuneBits == 0x1f0e9, "tuning bits");
+    // explicit: the bits the header defines (REVERSE, MARCH, PDL, TBLOCK,
+    // SC_STAGED, SC_NO_TMA, the block shape); any other bit is ignored
+    constexpr int kTuneBits = LB_TUNE_REVERSE | LB_TUNE_MARCH | LB_TUNE_PDL | LB_TUNE_TBLOCK |
+                              LB_TUNE_SC_STAGED | LB_TUNE_SC_NO_TMA | LB_TUNE_TBLOCK_SHAPE(0x1f);
+    static_assert(kTuneBits == 0x1f0eb, "tuning bits");
     c->tune = (cfg->tuning & LB_TUNE_EXPLICIT)
                   ? (cfg->tuning & kTuneBits)
                   : (cfg->lattice == LB_D2Q9 ? LB_TUNE_LIBRARY_DEFAULT_D2
@@ -444,6 +479,8 @@ int lb_create(const lb_config *cfg, lb_ctx **out) {
     if (!(cfg->tuning & LB_TUNE_EXPLICIT) && cfg->lattice == LB_D2Q9 &&
         N <= TBLOCK_DEFAULT_MAX_NODES)
         c->tune |= LB_TUNE_TBLOCK | LB_TUNE_TBLOCK_SHAPE(TBLOCK_DEFAULT_SHAPE);
+    if (!(cfg->tuning & LB_TUNE_EXPLICIT) && cfg->lattice == LB_D2Q9 && N > MARCH_DEFAULT_MIN_NODES)
+        c->tune |= LB_TUNE_MARCH;
     c->Q = cfg->lattice;
     c->N = N;
     c->stride = (N + 127) / 128 * 128;  // every population array starts on a 256-byte boundary
@@ -491,6 +528,7 @@ int lb_destroy(lb_ctx *c) {
         if (c->pop[i]) cudaFree(c->pop[i]);
     }
     if (c->flags) cudaFree(c->flags);
+    if (c->wmask) cudaFree(c->wmask);
     if (c->sb) cudaFree(c->sb);
     if (c->mom) cudaFree(c->mom);
     if (c->sc) cudaFree(c->sc);
@@ -527,6 +565,8 @@ int lb_set_flags(lb_ctx *c, const uint8_t *flags) {
     for (long o = 0; o < c->N && !any_wall; o++) any_wall = (f[o] & CELL_WALL) != 0;
     if (any_wall != c->any_wall) drop_graphs(c);  // the step kernel may change
     c->any_wall = any_wall;
+    const int rc = update_wall_mask(c, "lb_set_flags");
+    if (rc != LB_OK) return rc;
     return LB_OK;
 }
 
@@ -617,10 +657,10 @@ int lb_step(lb_ctx *c, int nsteps) {
         return fail(c, LB_ERR_STATE, "lb_step: a slab steps with lb_slab_step or "
                                      "lb_slab_group_step (its ghost planes need the exchange)");
     if (nsteps == 0) return LB_OK;
-    if (const int tv = tblock_variant(c)) {
-        // temporal blocks of T steps (graphs of L blocks); the last block, or
-        // the last per-step launch of a remainder, writes the moments
-        const int T = tblock_steps(tv), L = tblock_graph_launches(c, T);
+    if (const int T = multi_steps(c)) {
+        // launches of T steps (graphs of L launches); the last one, or the last
+        // per-step launch of a remainder, writes the moments
+        const int L = multi_graph_launches(c, T);
         int rest = nsteps;
         while (rest > L * T) {
             cudaGraphExec_t g;
@@ -631,8 +671,7 @@ int lb_step(lb_ctx *c, int nsteps) {
             rest -= L * T;
         }
         for (; rest >= T; rest -= T) {
-            LB_TRY(c, "lb_step", launch_d2q9_tblock(d2_args(c, c->cur), tv, rest == T, c->stream));
-            c->launches += 1;
+            LB_TRY(c, "lb_step", multi_once(c, c->cur, rest == T));
             c->cur = 1 - c->cur;
         }
         for (; rest > 0; rest--) {

@@ -156,6 +156,14 @@ cudaError_t launch_d2q9_fused_pdl(const D2Args &a, int mode, bool mom, cudaStrea
 // the moments of the last one.  tblock_steps is 0 for an unknown variant.
 int tblock_steps(int variant);
 cudaError_t launch_d2q9_tblock(const D2Args &a, int variant, bool mom, cudaStream_t s);
+// march_steps_per_launch() native steps (no Shan-Chen) in one pass, a.src to
+// a.dst, by warps that march down strips with the time levels in between in
+// registers (lb_march2d.cu), as a programmatic dependent launch; mask:
+// launch_d2q9_wall_mask's (N values, on 4 bytes), null on a lattice without walls
+int march_steps_per_launch();
+cudaError_t launch_d2q9_march(const D2Args &a, const uint16_t *mask, bool mom, cudaStream_t s);
+cudaError_t launch_d2q9_wall_mask(const uint8_t *flags, uint16_t *mask, int W, int H,
+                                  cudaStream_t s);
 cudaError_t launch_d2q9_stream_swap(const Pop<9> &p, const uint8_t *sb, int W, int H,
                                     cudaStream_t s);
 cudaError_t launch_d2q9_collide(const D2Args &a, bool plot, cudaStream_t s);
