@@ -574,6 +574,22 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         if (TRAIN) zn = v ? Z[s] : 0.f;
     };
     load_inputs((long)blockIdx.x * 128);
+    if (TRAIN) {
+        // the constant rows: ones (bias gradients) and zeros (padding)
+        constexpr uint32_t ONE = 0x3F80u;  // 1.0 in BF16
+        for (int r = ROW_ONES; r < 96; r++) st_b16(sGB, kmajor_offset(r, t, 128), r == ROW_ONES ? ONE : 0u);
+        for (int r = MLP_H; r < 128; r++) st_b16(sHA, kmajor_offset(r, t, 128), r == MLP_H ? ONE : 0u);
+        for (int r = 1; r < 16; r++) st_b16(sDY, kmajor_offset(r, t, 128), 0u);
+        if (t < 4) sloss[t] = 0.f;
+    }
+    if (t == 0) mbar_init(mbar, 1);
+    if (warp == 0) tc_alloc(tslot, NCOLS);
+    // everything above is ready while the previous launch (training: the
+    // reduction and Adam step) still runs; the weights are its result
+    if (TRAIN) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     // the weights in 16-byte pieces (8 BF16 of a row), all loads issued first:
     // W1 2 pieces per thread, W2 4 and, for training, W2^T 4
     {
@@ -611,16 +627,6 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         }
         if (t == 0) sw3[MLP_H] = bv3;
     }
-    if (TRAIN) {
-        // the constant rows: ones (bias gradients) and zeros (padding)
-        constexpr uint32_t ONE = 0x3F80u;  // 1.0 in BF16
-        for (int r = ROW_ONES; r < 96; r++) st_b16(sGB, kmajor_offset(r, t, 128), r == ROW_ONES ? ONE : 0u);
-        for (int r = MLP_H; r < 128; r++) st_b16(sHA, kmajor_offset(r, t, 128), r == MLP_H ? ONE : 0u);
-        for (int r = 1; r < 16; r++) st_b16(sDY, kmajor_offset(r, t, 128), 0u);
-        if (t < 4) sloss[t] = 0.f;
-    }
-    if (t == 0) mbar_init(mbar, 1);
-    if (warp == 0) tc_alloc(tslot, NCOLS);
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
@@ -877,6 +883,18 @@ __global__ void __launch_bounds__(RED_PAR * RED_RUNS)
     const int i = blockIdx.x * RED_PAR + pl;
     const int per = (nblocks + RED_RUNS - 1) / RED_RUNS;
     const int b0 = min(run * per, nblocks), b1 = min(b0 + per, nblocks);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the parameter and its moments: written last by the reduction before, which
+    // was complete before the training kernel let this launch start (through L2:
+    // this SM's L1 may hold older lines)
+    const bool adam = ad.p && run == 0 && i < MLP_NPARAM;
+    float p0 = 0.f, a0 = 0.f, q0 = 0.f;
+    if (adam) {
+        p0 = __ldcg(ad.p + i);
+        a0 = __ldcg(ad.m1 + i);
+        q0 = __ldcg(ad.m2 + i);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     float s = 0.f;
     if (i < NGRAD) {
         int b = b0;
@@ -900,12 +918,12 @@ __global__ void __launch_bounds__(RED_PAR * RED_RUNS)
         if (loss_slot) *loss_slot = s;
         return;
     }
-    if (!ad.p) return;
-    const float a = 0.9f * ad.m1[i] + 0.1f * s;
-    const float q = 0.999f * ad.m2[i] + 0.001f * s * s;
+    if (!adam) return;
+    const float a = 0.9f * a0 + 0.1f * s;
+    const float q = 0.999f * q0 + 0.001f * s * s;
     ad.m1[i] = a;
     ad.m2[i] = q;
-    const float v = ad.p[i] - ad.lr * (a / ad.b1c) / (sqrtf(q / ad.b2c) + 1e-8f);
+    const float v = p0 - ad.lr * (a / ad.b1c) / (sqrtf(q / ad.b2c) + 1e-8f);
     ad.p[i] = v;
     if (i < MLP_OFF_B1)
         ad.w1b[(i / MLP_IN) * MLP_IN_PAD + i % MLP_IN] = __float2bfloat16_rn(v);
@@ -996,12 +1014,25 @@ int mlp_gradient(lb_mlp *m, const float *X, const float *Z, long n, float *loss_
     LB_MTRY(m, "cudaFuncSetAttribute", mlp_kernel_attributes());
     const long chunks = (n + 127) / 128;
     const int nb = (int)std::min<long>(m->nblocks, chunks);
-    mlp_tc_kernel<true><<<nb, 128, net::TRAIN_SMEM, m->stream>>>(mlp_dev(m), X, Z, n, m->partial,
-                                                                 m->err_dev);
-    LB_MTRY(m, "mlp_tc_kernel", cudaGetLastError());
-    grad_reduce_kernel<<<(NGRAD + RED_PAR - 1) / RED_PAR, RED_PAR * RED_RUNS, 0, m->stream>>>(
-        m->partial, nb, m->grad, loss_slot, ad);
-    LB_MTRY(m, "grad_reduce_kernel", cudaGetLastError());
+    // both as programmatic dependents of the launch before them
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = net::TRAIN_SMEM;
+    cfg.stream = m->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LB_MTRY(m, "mlp_tc_kernel", cudaLaunchKernelEx(&cfg, mlp_tc_kernel<true>, mlp_dev(m), X, Z, n,
+                                                   m->partial, m->err_dev));
+    cfg.gridDim = dim3((NGRAD + RED_PAR - 1) / RED_PAR);
+    cfg.blockDim = dim3(RED_PAR * RED_RUNS);
+    cfg.dynamicSmemBytes = 0;
+    LB_MTRY(m, "grad_reduce_kernel", cudaLaunchKernelEx(&cfg, grad_reduce_kernel,
+                                                        (const float *)m->partial, nb, m->grad,
+                                                        loss_slot, ad));
     return LB_OK;
 }
 
