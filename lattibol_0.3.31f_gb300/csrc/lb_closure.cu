@@ -478,8 +478,13 @@ __global__ void features_kernel(const float *fl, int Wc, int Hc, int Dc, float n
 // The network's forward pass and, for training, its backward pass over tiles
 // of 128 samples on the 5th-generation tensor cores.  Thread t owns sample t
 // of a tile, row t of the sample-major MMA tiles, column t of the transposed
-// (sample-contracted) tiles and lane t of tensor memory.  Thread 0 issues
-// every MMA (BF16 operands in shared memory, K-major core matrices,
+// (sample-contracted) tiles and lane t of tensor memory; in training threads t
+// and t + 128 share them, each with half of the hidden columns (the launch is
+// one tile per block, a latency chain of five MMA groups and the epilogues
+// between them: half as many columns per thread, and block sums stored in rows
+// of consecutive floats, took a step of 16 384 samples from 14.2 to 10.9 us;
+// 20.2 before the launches overlapped).  The output's sum over all 64 columns
+// is formed by both, in the one order.  Thread 0 issues every MMA (BF16 operands in shared memory, K-major core matrices,
 // lb_tc05.cuh; FP32 accumulators in tensor memory) and commits it to one
 // mbarrier.  Per tile:
 //   1. x (19 features, padded to 32) -> row t of A; D_h1 = A W1^T;
@@ -523,6 +528,24 @@ static_assert(OFF_F % 16 == 0 && OFF_GA % 16 == 0 && OFF_GB % 16 == 0 && OFF_HA 
 static_assert(COL_G3 + 16 <= 256 && ROW_ONES < 96, "tensor-memory and tile extents");
 }  // namespace net
 constexpr int NGRAD = MLP_NPARAM + 1;  // + loss
+// A block's sums: the parameters' gradients with the accumulator row j fastest,
+// so that a warp's stores (one row per lane) and the reduction's loads are
+// contiguous (in the parameters' own order each store touched 32 sectors).
+constexpr int SUM_W2 = 0;                          // [column c][row j]: dW2[j][c]
+constexpr int SUM_W1 = SUM_W2 + MLP_H * MLP_H;     // [input f][row j]: dW1[j][f]
+constexpr int SUM_B1 = SUM_W1 + MLP_IN * MLP_H, SUM_B2 = SUM_B1 + MLP_H;
+constexpr int SUM_W3 = SUM_B2 + MLP_H, SUM_B3 = SUM_W3 + MLP_H, SUM_LOSS = SUM_B3 + 1;
+static_assert(SUM_LOSS + 1 == NGRAD, "one sum per parameter, and the loss");
+// the parameter (or, last, the loss) of sum i
+__device__ __forceinline__ int sum_param(int i) {
+    if (i < SUM_W1) return MLP_OFF_W2 + (i % MLP_H) * MLP_H + i / MLP_H;
+    if (i < SUM_B1) return MLP_OFF_W1 + (i % MLP_H) * MLP_IN + (i - SUM_W1) / MLP_H;
+    if (i < SUM_B2) return MLP_OFF_B1 + i - SUM_B1;
+    if (i < SUM_W3) return MLP_OFF_B2 + i - SUM_B2;
+    if (i < SUM_B3) return MLP_OFF_W3 + i - SUM_W3;
+    return i == SUM_B3 ? MLP_OFF_B3 : MLP_NPARAM;
+}
+static_assert(SUM_W1 % MLP_H == 0, "i % 64 is the row");
 constexpr int NET_FWD_SMEM = 50 * 1024;  // at most 4 blocks (4 x 128 columns) per SM
 
 __device__ __forceinline__ void st_b16(uint8_t *base, uint32_t off, uint32_t bits) {
@@ -549,7 +572,7 @@ __device__ __forceinline__ void st_col4(uint8_t *tile, int r0, int t, uint32_t w
 }
 
 template <bool TRAIN>
-__global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const float *X,
+__global__ void __launch_bounds__(TRAIN ? 256 : 128, 1) mlp_tc_kernel(const MlpDev mlp, const float *X,
                                                      const float *Z, long n, float *out,
                                                      int *err) {
     using namespace net;
@@ -561,71 +584,79 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
     float *sloss = sw3 + MLP_H + 1;  // after b3: one sum per warp
     uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + OFF_F + 800);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + OFF_F + 808);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    // training: two threads per sample, one for each half of the columns
+    constexpr int HALVES = TRAIN ? 2 : 1;
+    constexpr int XN = TRAIN ? 16 : MLP_IN;     // features of a thread
+    constexpr int CW = MLP_H / HALVES;          // hidden columns of a thread
+    const int tid = threadIdx.x, t = tid & 127, warp = t >> 5, lane = t & 31;
+    const int half = TRAIN ? tid >> 7 : 0, c0 = half * CW, x0 = half * XN;
 
     // the first tile's inputs are loaded before the weights are staged, every
     // later tile's while the MMAs of the one before run
-    float x[MLP_IN], zn = 0.f;
+    float x[XN], zn = 0.f;
     auto load_inputs = [&](long b) {
         const long s = b + t;
         const bool v = s < n;
 #pragma unroll
-        for (int i = 0; i < MLP_IN; i++) x[i] = v ? X[s * MLP_IN + i] : 0.f;
+        for (int i = 0; i < XN; i++)
+            x[i] = v && (!TRAIN || x0 + i < MLP_IN) ? X[s * MLP_IN + x0 + i] : 0.f;
         if (TRAIN) zn = v ? Z[s] : 0.f;
     };
     load_inputs((long)blockIdx.x * 128);
     if (TRAIN) {
         // the constant rows: ones (bias gradients) and zeros (padding)
         constexpr uint32_t ONE = 0x3F80u;  // 1.0 in BF16
-        for (int r = ROW_ONES; r < 96; r++) st_b16(sGB, kmajor_offset(r, t, 128), r == ROW_ONES ? ONE : 0u);
-        for (int r = MLP_H; r < 128; r++) st_b16(sHA, kmajor_offset(r, t, 128), r == MLP_H ? ONE : 0u);
-        for (int r = 1; r < 16; r++) st_b16(sDY, kmajor_offset(r, t, 128), 0u);
-        if (t < 4) sloss[t] = 0.f;
+        for (int r = ROW_ONES + half; r < 96; r += 2)
+            st_b16(sGB, kmajor_offset(r, t, 128), r == ROW_ONES ? ONE : 0u);
+        for (int r = MLP_H + half; r < 128; r += 2)
+            st_b16(sHA, kmajor_offset(r, t, 128), r == MLP_H ? ONE : 0u);
+        for (int r = 1 + half; r < 16; r += 2) st_b16(sDY, kmajor_offset(r, t, 128), 0u);
+        if (tid < 4) sloss[tid] = 0.f;
     }
-    if (t == 0) mbar_init(mbar, 1);
-    if (warp == 0) tc_alloc(tslot, NCOLS);
+    if (tid == 0) mbar_init(mbar, 1);
+    if (tid < 32) tc_alloc(tslot, NCOLS);
     // everything above is ready while the previous launch (training: the
     // reduction and Adam step) still runs; the weights are its result
     if (TRAIN) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
-    // the weights in 16-byte pieces (8 BF16 of a row), all loads issued first:
-    // W1 2 pieces per thread, W2 4 and, for training, W2^T 4
+    // the weights in 16-byte pieces (8 BF16 of a row), all loads issued first
     {
+        constexpr int NT = 128 * HALVES, N1 = 256 / NT, N2 = 512 / NT;
         const uint4 *w1v = reinterpret_cast<const uint4 *>(mlp.w1);
         const uint4 *w2v = reinterpret_cast<const uint4 *>(mlp.w2);
         const uint4 *w2tv = reinterpret_cast<const uint4 *>(mlp.w2t);
-        uint4 p1[2], p2[4], p3[4];
+        uint4 p1[N1], p2[N2], p3[N2];
 #pragma unroll
-        for (int u = 0; u < 2; u++) p1[u] = w1v[t + 128 * u];
+        for (int u = 0; u < N1; u++) p1[u] = w1v[tid + NT * u];
 #pragma unroll
-        for (int u = 0; u < 4; u++) p2[u] = w2v[t + 128 * u];
+        for (int u = 0; u < N2; u++) p2[u] = w2v[tid + NT * u];
         if (TRAIN) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) p3[u] = w2tv[t + 128 * u];
+            for (int u = 0; u < N2; u++) p3[u] = w2tv[tid + NT * u];
         }
-        const float bv1 = t < MLP_H ? mlp.b1[t] : 0.f, bv2 = t < MLP_H ? mlp.b2[t] : 0.f;
-        const float wv3 = t < MLP_H ? mlp.w3[t] : 0.f, bv3 = mlp.b3[0];
+        const float bv1 = tid < MLP_H ? mlp.b1[tid] : 0.f, bv2 = tid < MLP_H ? mlp.b2[tid] : 0.f;
+        const float wv3 = tid < MLP_H ? mlp.w3[tid] : 0.f, bv3 = mlp.b3[0];
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int q = t + 128 * u;  // row q / 4, columns 8 (q % 4) ..
+        for (int u = 0; u < N1; u++) {
+            const int q = tid + NT * u;  // row q / 4, columns 8 (q % 4) ..
             *reinterpret_cast<uint4 *>(smem + OFF_W1 +
                                        kmajor_offset(q / 4, 8 * (q % 4), MLP_IN_PAD)) = p1[u];
         }
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int q = t + 128 * u, j = q / 8, k0 = 8 * (q % 8);  // row j, columns k0 ..
+        for (int u = 0; u < N2; u++) {
+            const int q = tid + NT * u, j = q / 8, k0 = 8 * (q % 8);  // row j, columns k0 ..
             *reinterpret_cast<uint4 *>(smem + OFF_W2 + kmajor_offset(j, k0, MLP_H)) = p2[u];
             if (TRAIN)
                 *reinterpret_cast<uint4 *>(smem + OFF_W2T + kmajor_offset(j, k0, MLP_H)) = p3[u];
         }
-        if (t < MLP_H) {
-            sb1[t] = bv1;
-            sb2[t] = bv2;
-            sw3[t] = wv3;
+        if (tid < MLP_H) {
+            sb1[tid] = bv1;
+            sb2[tid] = bv2;
+            sw3[tid] = wv3;
         }
-        if (t == 0) sw3[MLP_H] = bv3;
+        if (tid == 0) sw3[MLP_H] = bv3;
     }
     fence_proxy_async();
     tc_fence_before();
@@ -648,12 +679,12 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
-        if (t == 0) {
+        if (tid == 0) {
             tc_fence_after();
             issue();
             tc_commit(mbar);
         }
-        const bool done = __syncthreads_and(t == 0 ? mbar_wait(mbar, phase, TC_WAIT) : true);
+        const bool done = __syncthreads_and(tid == 0 ? mbar_wait(mbar, phase, TC_WAIT) : true);
         phase ^= 1;
         tc_fence_after();
         return done;
@@ -667,21 +698,24 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         const float zv = zn;
         // 1. x -> row t of A (K 32); training: column t of X^T
 #pragma unroll
-        for (int h = 0; h < MLP_IN_PAD / 8; h++) {
+        for (int h = 0; h < MLP_IN_PAD / 8 / HALVES; h++) {
             uint32_t p[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int k0 = 8 * h + 2 * j;
-                p[j] = bf16x2_bits(k0 < MLP_IN ? x[k0] : 0.f, k0 + 1 < MLP_IN ? x[k0 + 1] : 0.f);
+                p[j] = bf16x2_bits(k0 < XN ? x[k0] : 0.f, k0 + 1 < XN ? x[k0 + 1] : 0.f);
             }
-            // rows 64 + k of [H1^T; X^T; 1; 0]: features 0-18, then the row of ones
+            // rows 64 + k of [H1^T; X^T; 1; 0]: features 0-18, then the row of ones,
+            // which closes the features' last group of 4
             constexpr uint32_t ONE_HI = 0x3F800000u;  // BF16 1.0 in the high half
-            static_assert(MLP_IN % 4 == 3, "the row of ones closes the features' last group of 4");
-            if (TRAIN && 8 * h < MLP_IN)
-                st_col4(sGB, MLP_H + 8 * h, t, p[0], 8 * h + 3 == MLP_IN ? p[1] | ONE_HI : p[1]);
-            if (TRAIN && 8 * h + 4 < MLP_IN)
-                st_col4(sGB, MLP_H + 8 * h + 4, t, p[2], 8 * h + 7 == MLP_IN ? p[3] | ONE_HI : p[3]);
-            *reinterpret_cast<uint4 *>(sA + kmajor_offset(t, 8 * h, MLP_IN_PAD)) =
+            static_assert(!TRAIN || (XN == 16 && MLP_IN == 19), "the halves' features");
+            if (TRAIN && half == 0) {
+                st_col4(sGB, MLP_H + 8 * h, t, p[0], p[1]);
+                st_col4(sGB, MLP_H + 8 * h + 4, t, p[2], p[3]);
+            } else if (TRAIN && h == 0) {
+                st_col4(sGB, MLP_H + XN, t, p[0], p[1] | ONE_HI);
+            }
+            *reinterpret_cast<uint4 *>(sA + kmajor_offset(t, x0 + 8 * h, MLP_IN_PAD)) =
                 make_uint4(p[0], p[1], p[2], p[3]);
         }
         if (base + (long)gridDim.x * 128 < n) load_inputs(base + (long)gridDim.x * 128);
@@ -694,9 +728,10 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         if (!ok) break;
         // 2. h1 = ReLU(D + b1) as BF16 -> row t of A (K 64); training: column t
         // of H1^T and the mask h1 > 0
-        uint64_t m1 = 0;
+        uint32_t m1 = 0;  // training: of the thread's own 32 columns
 #pragma unroll
-        for (int c = 0; c < MLP_H; c += 32) {
+        for (int cc = 0; cc < CW; cc += 32) {
+            const int c = c0 + cc;
             float v[32];
             tc_ld32(lane_base + COL_H1 + (uint32_t)c, v);
 #pragma unroll
@@ -709,8 +744,8 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
                                                  make_float2(sb1[c + q], sb1[c + q + 1]));
                     p[j] = bf16x2_relu(hv.x, hv.y);
                     if (TRAIN) {
-                        m1 |= (uint64_t)((p[j] & 0xFFFFu) != 0u) << (c + q);
-                        m1 |= (uint64_t)((p[j] >> 16) != 0u) << (c + q + 1);
+                        m1 |= (uint32_t)((p[j] & 0xFFFFu) != 0u) << q;
+                        m1 |= (uint32_t)((p[j] >> 16) != 0u) << (q + 1);
                     }
                 }
                 if (TRAIN) {
@@ -754,12 +789,14 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         float e2 = e * e;
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, d);
-        if (lane == 0) sloss[warp] += e2;
-        st_b16(sDY, kmajor_offset(0, t, 128), bf16x2_bits(dy, 0.f));
+        if (half == 0) {
+            if (lane == 0) sloss[warp] += e2;
+            st_b16(sDY, kmajor_offset(0, t, 128), bf16x2_bits(dy, 0.f));
+        }
         // dH2 = dy w3 (h2 > 0) as BF16 -> row t of A and column t of dH2^T;
-        // h2 as BF16 -> column t of H2^T
-#pragma unroll
-        for (int c = 0; c < MLP_H; c += 32) {
+        // h2 as BF16 -> column t of H2^T (each thread its half of the columns)
+        {
+            const int c = c0;
             float v[32];
             tc_ld32(lane_base + COL_H2 + (uint32_t)c, v);
 #pragma unroll
@@ -792,16 +829,16 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         });
         if (!ok) break;
         // 4. dH1 = D (h1 > 0) as BF16 -> column t of dH1^T
-#pragma unroll
-        for (int c = 0; c < MLP_H; c += 32) {
+        {
+            const int c = c0;
             float v[32];
             tc_ld32(lane_base + COL_H1 + (uint32_t)c, v);
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
-                const uint32_t p01 = bf16x2_bits((m1 >> (c + j)) & 1 ? v[j] : 0.f,
-                                                 (m1 >> (c + j + 1)) & 1 ? v[j + 1] : 0.f);
-                const uint32_t p23 = bf16x2_bits((m1 >> (c + j + 2)) & 1 ? v[j + 2] : 0.f,
-                                                 (m1 >> (c + j + 3)) & 1 ? v[j + 3] : 0.f);
+                const uint32_t p01 = bf16x2_bits((m1 >> j) & 1 ? v[j] : 0.f,
+                                                 (m1 >> (j + 1)) & 1 ? v[j + 1] : 0.f);
+                const uint32_t p23 = bf16x2_bits((m1 >> (j + 2)) & 1 ? v[j + 2] : 0.f,
+                                                 (m1 >> (j + 3)) & 1 ? v[j + 3] : 0.f);
                 st_col4(sGA, MLP_H + c + j, t, p01, p23);
             }
         }
@@ -819,45 +856,48 @@ __global__ void __launch_bounds__(128, 1) mlp_tc_kernel(const MlpDev mlp, const 
         if (!ok) break;
     }
     if (TRAIN && ok) {
-        // the block's sums: warps 0-1 hold rows j of dW2, db2 and dw3, warps
-        // 2-3 rows i of dW1 and db1, lane 64 db3
+        // the block's sums in the order of NetSums: rows 0-63 of the accumulators
+        // (t < 64) hold dW2, db2 and dw3, rows 64-127 dW1 and db1, row 64 db3;
+        // the threads' halves take half of the columns each
         float *pb = out + (long)blockIdx.x * NGRAD;
         float v[32];
         if (ntile == 0) {
-            for (int i = t; i < NGRAD; i += 128) pb[i] = 0.f;
+            for (int i = tid; i < NGRAD; i += 256) pb[i] = 0.f;
         } else {
+            const int j = t & 63;
             if (warp < 2) {
+                tc_ld32(lane_base + COL_G + (uint32_t)c0, v);
 #pragma unroll
-                for (int c = 0; c < MLP_H; c += 32) {
-                    tc_ld32(lane_base + COL_G + (uint32_t)c, v);
+                for (int i = 0; i < 32; i++) pb[SUM_W2 + (c0 + i) * MLP_H + j] = v[i];
+            }
+            if (half == 0) {
+                tc_ld32(lane_base + COL_G + MLP_H, v);
+                if (warp < 2) {
+                    pb[SUM_B2 + j] = v[MLP_IN];
+                } else {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) pb[MLP_OFF_W2 + t * MLP_H + c + i] = v[i];
+                    for (int f = 0; f < MLP_IN; f++) pb[SUM_W1 + f * MLP_H + j] = v[f];
+                    pb[SUM_B1 + j] = v[MLP_IN];
                 }
-            }
-            tc_ld32(lane_base + COL_G + MLP_H, v);
-            if (warp < 2) {
-                pb[MLP_OFF_B2 + t] = v[MLP_IN];
             } else {
-#pragma unroll
-                for (int f = 0; f < MLP_IN; f++) pb[MLP_OFF_W1 + (t - MLP_H) * MLP_IN + f] = v[f];
-                pb[MLP_OFF_B1 + t - MLP_H] = v[MLP_IN];
+                tc_ld32(lane_base + COL_G3, v);
+                if (warp < 2) pb[SUM_W3 + j] = v[0];
+                else if (t == MLP_H) pb[SUM_B3] = v[0];
             }
-            tc_ld32(lane_base + COL_G3, v);
-            if (t < MLP_H) pb[MLP_OFF_W3 + t] = v[0];
-            else if (t == MLP_H) pb[MLP_OFF_B3] = v[0];
-            if (t == 0) pb[MLP_NPARAM] = ((sloss[0] + sloss[1]) + (sloss[2] + sloss[3])) * inv_n;
+            if (tid == 0)
+                pb[SUM_LOSS] = ((sloss[0] + sloss[1]) + (sloss[2] + sloss[3])) * inv_n;
         }
     }
     if (!ok) {
         // an MMA did not complete: record it, give it one more bounded wait so
         // that no MMA is writing the columns when they are released
-        if (t == 0 && err) atomicExch(err, 1);
+        if (tid == 0 && err) atomicExch(err, 1);
         mbar_wait(mbar, phase ^ 1, TC_WAIT);
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, NCOLS);
-    if (t == 0) mbar_inval(mbar);
+    if (tid < 32) tc_dealloc(tmem, NCOLS);
+    if (tid == 0) mbar_inval(mbar);
 }
 
 // one Adam step of the FP32 master parameters (p == nullptr: none)
@@ -880,7 +920,8 @@ __global__ void __launch_bounds__(RED_PAR * RED_RUNS)
                        const AdamStep ad) {
     __shared__ float run_sum[RED_RUNS][RED_PAR];
     const int pl = threadIdx.x % RED_PAR, run = threadIdx.x / RED_PAR;
-    const int i = blockIdx.x * RED_PAR + pl;
+    const int si = blockIdx.x * RED_PAR + pl;       // the sum, and its parameter
+    const int i = si < NGRAD ? sum_param(si) : NGRAD;
     const int per = (nblocks + RED_RUNS - 1) / RED_RUNS;
     const int b0 = min(run * per, nblocks), b1 = min(b0 + per, nblocks);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -901,11 +942,11 @@ __global__ void __launch_bounds__(RED_PAR * RED_RUNS)
         for (; b + 16 <= b1; b += 16) {
             float v[16];
 #pragma unroll
-            for (int u = 0; u < 16; u++) v[u] = partial[(long)(b + u) * NGRAD + i];
+            for (int u = 0; u < 16; u++) v[u] = partial[(long)(b + u) * NGRAD + si];
 #pragma unroll
             for (int u = 0; u < 16; u++) s = s + v[u];
         }
-        for (; b < b1; b++) s = s + partial[(long)b * NGRAD + i];
+        for (; b < b1; b++) s = s + partial[(long)b * NGRAD + si];
     }
     run_sum[run][pl] = s;
     __syncthreads();
@@ -1020,7 +1061,7 @@ int mlp_gradient(lb_mlp *m, const float *X, const float *Z, long n, float *loss_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nb);
-    cfg.blockDim = dim3(128);
+    cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = net::TRAIN_SMEM;
     cfg.stream = m->stream;
     cfg.attrs = attr;
