@@ -41,7 +41,8 @@ struct lb_ctx {
     float corr[19] = {0};
     float wr[19] = {0};                  // 16-bit storage offsets w_k * rho_ref
     int tune = 0;                        // LB_TUNE_* bits in effect
-    uint16_t *wmask = nullptr;           // marching strips: upstream-wall masks
+    MarchPlan march{};                   // marching strips: the items of a launch
+    uint16_t *wmask = nullptr;           // and their upstream-wall masks
     bool closure_on = false;             // learned closure sets the local relaxation time
     ClosureArgs closure{};
     bool flags_set = false;
@@ -338,8 +339,8 @@ cudaError_t step_once(lb_ctx *c, int from, bool moments) {
 cudaError_t multi_once(lb_ctx *c, int from, bool moments) {
     c->launches += 1;
     if (march_on(c))
-        return launch_d2q9_march(d2_args(c, from), c->any_wall ? c->wmask : nullptr, moments,
-                                 c->stream);
+        return launch_d2q9_march(d2_args(c, from), c->march, c->any_wall ? c->wmask : nullptr,
+                                 moments, c->stream);
     return launch_d2q9_tblock(d2_args(c, from), tblock_variant(c), moments, c->stream);
 }
 
@@ -414,17 +415,25 @@ void prepare_flags(const lb_ctx *c, const uint8_t *in, std::vector<uint8_t> &fla
         any_wall = any_wall || flags[o];
     }
     if (!any_wall) return;  // fully periodic: no fluid cell is near a wall
+    // away from the lattice's faces a neighbour is at a fixed distance in memory
+    long dist[19];
+    for (int k = 0; k < Q; k++)
+        dist[k] = Q == 19 ? d3_cx(k) + (long)W * (d3_cy(k) + (long)H * d3_cz(k))
+                          : d2_cx(k) + (long)W * d2_cr(k);
     for (int z = 0; z < D; z++)
-        for (int y = 0; y < H; y++)
+        for (int y = 0; y < H; y++) {
+            const bool inner = y > 0 && y < H - 1 && (Q == 9 || (z > 0 && z < D - 1));
             for (int x = 0; x < W; x++) {
                 const long o = x + (long)W * (y + (long)H * z);
                 if (flags[o] & CELL_WALL) continue;
+                const bool near = inner && x > 0 && x < W - 1;
                 for (int k = 1; k < Q; k++)
-                    if (flags[nb(x, y, z, k, true)] & CELL_WALL) {
+                    if (flags[near ? o + dist[k] : nb(x, y, z, k, true)] & CELL_WALL) {
                         flags[o] |= CELL_NEAR_WALL;
                         break;
                     }
             }
+        }
 }
 
 }  // namespace
@@ -483,6 +492,7 @@ int lb_create(const lb_config *cfg, lb_ctx **out) {
         c->tune |= LB_TUNE_MARCH;
     c->Q = cfg->lattice;
     c->N = N;
+    if (c->tune & LB_TUNE_MARCH) c->march = march_plan(cfg->nx, cfg->ny);
     c->stride = (N + 127) / 128 * 128;  // every population array starts on a 256-byte boundary
     c->esize = cfg->storage == LB_STORE_F32 ? 4 : 2;
     wall_corr(c->cfg, c->corr);

@@ -160,8 +160,13 @@ cudaError_t launch_d2q9_tblock(const D2Args &a, int variant, bool mom, cudaStrea
 // a.dst, by warps that march down strips with the time levels in between in
 // registers (lb_march2d.cu), as a programmatic dependent launch; mask:
 // launch_d2q9_wall_mask's (N values, on 4 bytes), null on a lattice without walls
+struct MarchPlan {
+    int tw, rows, strips, items;  // columns and rows of an item; strips; items
+};
+MarchPlan march_plan(int W, int H);
 int march_steps_per_launch();
-cudaError_t launch_d2q9_march(const D2Args &a, const uint16_t *mask, bool mom, cudaStream_t s);
+cudaError_t launch_d2q9_march(const D2Args &a, const MarchPlan &p, const uint16_t *mask, bool mom,
+                              cudaStream_t s);
 cudaError_t launch_d2q9_wall_mask(const uint8_t *flags, uint16_t *mask, int W, int H,
                                   cudaStream_t s);
 cudaError_t launch_d2q9_stream_swap(const Pop<9> &p, const uint8_t *sb, int W, int H,

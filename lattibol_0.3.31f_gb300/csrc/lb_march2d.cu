@@ -49,7 +49,7 @@ constexpr uint32_t MD_NEAR = 0x00ff00ffu;  // wall bits of a mask pair
 struct MarchArgs {
     D2Args a;
     const uint16_t *mask;
-    int tw, rows, strips, items;
+    int tw, rows, strips, items;  // MarchPlan
     PairConst c;
     PairD2 d;
 };
@@ -285,28 +285,8 @@ cudaError_t launch_d2q9_wall_mask(const uint8_t *flags, uint16_t *mask, int W, i
 namespace {
 
 template <bool MOM, bool WALLS>
-cudaError_t md_launch(MarchArgs &ma, cudaStream_t s) {
+cudaError_t md_launch(const MarchArgs &ma, cudaStream_t s) {
     const D2Args &a = ma.a;
-    const int ns = (a.W + MD_COLS - 1) / MD_COLS;
-    ma.tw = ((a.W + ns - 1) / ns + 3) & ~3;
-    ma.strips = (a.W + ma.tw - 1) / ma.tw;
-    // Rows per item: fewer rows fill the GPU's warps, more rows pay less for the
-    // 2 T rows that an item reads beyond its own.  A pass takes an item's march
-    // times the rounds of items; a partly filled round runs its warps faster
-    // (measured at 1568 x 1024: 16 rows, 1792 items for 1824 warps, 1.20 ms per
-    // 100 steps; 12 rows 1.48, 24 rows 1.41, 32 rows 1.68).
-    const double warps = 152. * MD_BLOCKS;
-    double best = 0;
-    for (int c = 1; c <= a.H; c++) {
-        const int r = (a.H + c - 1) / c;
-        const double w = ma.strips * (double)((a.H + r - 1) / r) / warps;
-        const double cost = (r + 2. * T) * (w <= 1. ? 0.65 + 0.35 * w : w + 0.25);
-        if (best == 0 || cost < best) {
-            best = cost;
-            ma.rows = r;
-        }
-    }
-    ma.items = ma.strips * ((a.H + ma.rows - 1) / ma.rows);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ma.items);
     cfg.blockDim = dim3(32);
@@ -326,10 +306,42 @@ cudaError_t md_launch(MarchArgs &ma, cudaStream_t s) {
 
 int march_steps_per_launch() { return T; }
 
-cudaError_t launch_d2q9_march(const D2Args &a, const uint16_t *mask, bool mom, cudaStream_t s) {
+// Rows per item: fewer rows fill the GPU's warps, more rows pay less for the 2 T
+// rows that an item reads beyond its own.  A pass takes an item's march times a
+// function of the rounds of items w (a partly filled round runs its warps
+// faster, a nearly empty second one costs almost as much as a full one;
+// measured at 1568 x 1024: 16 rows, 1792 items for 1824 warps, 1.20 ms per 100
+// steps; 12 rows 1.48, 24 rows 1.41, 32 rows 1.68).
+MarchPlan march_plan(int W, int H) {
+    MarchPlan p{};
+    const int ns = (W + MD_COLS - 1) / MD_COLS;
+    p.tw = ((W + ns - 1) / ns + 3) & ~3;
+    p.strips = (W + p.tw - 1) / p.tw;
+    const double warps = 152. * MD_BLOCKS;
+    double best = 0;
+    for (int c = 1; c <= H; c++) {
+        const int r = (H + c - 1) / c;
+        const double w = p.strips * (double)((H + r - 1) / r) / warps;
+        const double cost =
+            (r + 2. * T) * (w <= 1. ? 0.65 + 0.35 * w : std::max(1.42, 0.32 + 0.82 * w));
+        if (best == 0 || cost < best) {
+            best = cost;
+            p.rows = r;
+        }
+    }
+    p.items = p.strips * ((H + p.rows - 1) / p.rows);
+    return p;
+}
+
+cudaError_t launch_d2q9_march(const D2Args &a, const MarchPlan &p, const uint16_t *mask, bool mom,
+                              cudaStream_t s) {
     if (a.G != 0.f) return cudaErrorInvalidValue;  // no Shan-Chen here
     MarchArgs ma{};
     ma.a = a;
+    ma.tw = p.tw;
+    ma.rows = p.rows;
+    ma.strips = p.strips;
+    ma.items = p.items;
     ma.mask = mask;
     ma.c = pair_constants();
     const auto two = [](float v) { return make_float2(v, v); };
