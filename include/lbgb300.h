@@ -263,8 +263,8 @@ int lb_wall_correction(const lb_ctx *ctx, float *corr);
 /* ======================================================================== */
 /* Many small lattices of different sizes advanced together: one packed
  * population slab (domain d at nodes [offset(d), offset(d) + nx[d]*ny[d]),
- * node x + nx[d]*y inside it), two persistent launches per step over a work
- * list of row groups, batches replayed from a captured CUDA graph.  Each
+ * node x + nx[d]*y inside it), launches over a work list of strips or row
+ * groups, batches replayed from a captured CUDA graph.  Each
  * domain is periodic, without walls or body force, with its own G and
  * tau_inv; a domain evolves bit for bit like the same lattice run alone
  * through the context API (native mode, same psi form). */
@@ -287,11 +287,11 @@ int lb_ensemble_get_moments(lb_ensemble *e, float *rho, float *ux, float *uy);
  * (1: 32 x 8 at 48 registers; 2: 32 x 8 at 40; 3: 32 x 16 at 60; 4: 32 x 16
  * at 40; 5: 32 x 32 at 60), 6..9 warps marching down 32-column strips with
  * psi of three rows in registers (6: 32 rows at 80 registers; 7: 32 rows at
- * 64; 8: 64 rows; 9: 16 rows), 10..12 the same strips fed by a per-warp
- * shared-memory ring of source rows copied ahead with cp.async (10: 32 rows,
- * the default with 3 blocks per SM; 11: 64 rows; 12: 16 rows; domains not a
- * multiple of 32 wide, or not starting on a 16-byte boundary, take the plain
- * strips).  Otherwise the two-pass step (psi pass, fused pass)
+ * 64; 8: 64 rows; 9: 16 rows), 10..12 strips of column
+ * pairs, two nodes per lane (10, the default: rows per strip of the library's
+ * choice, and two steps per launch on ensembles of 2^20 nodes and more whose
+ * domains' rows mostly start on 16 bytes; 11: 64 rows; 12: 16 rows; blocks per
+ * SM do not apply).  Otherwise the two-pass step (psi pass, fused pass)
  * over groups of `rows` rows with threads_x threads along x (a multiple of
  * 32).  Both give the same bits.  The autotuner times every candidate for
  * trial_steps steps on the ensemble itself (advancing its state: tune before

@@ -24,7 +24,7 @@
 #include <vector>
 
 #include "../../include/lbgb300.h"
-#include "lb_kernels.cuh"
+#include "lb_pairs.cuh"
 
 using namespace lb;
 
@@ -301,181 +301,208 @@ __global__ void __launch_bounds__(ENS_MARCH_THREADS, MINB) ens_march_kernel(cons
 }
 
 // ---------------------------------------------------------------------------
-// Strips with a shared-memory row ring.  The march above must wait for the
-// loads of row r + 1 before it can relax row r: a DRAM latency per row for
-// every warp.  Here each warp keeps the source rows its pulls read in a ring
-// of ENS_RING slots in shared memory (9 populations x 40 columns: the strip,
-// the two halo columns and their outer neighbours, rounded out to 16-byte
-// chunks) and copies source row r + 4 with 16-byte cp.async (one commit group
-// per row) before it pulls row r + 1, so rows land two rows ahead of their
-// use and the pulls are shared-memory loads.  A lane waits for its own groups
-// (cp.async.wait_group) and a warp barrier makes every lane's copies visible;
-// no block barrier.  An item qualifies when its domain's rows start on 16
-// bytes and no chunk straddles its periodic x edge (W a multiple of 32, first
-// node a multiple of 4); the work list puts those first, and the other items
-// take the plain march in a second launch (kept out of this kernel, whose
-// registers it would crowd).  Same pulls and arithmetic as the march, so the
-// same bits.
+// Strips of column pairs, one or two steps per launch.  A warp marches down a
+// strip of 64 columns, two per lane, both through the paired FP32 instructions
+// (lb_pairs.cuh; every lane the scalar operations in the scalar order, so the
+// same bits).  Input rows arrive in a ring of four per warp by 16-byte cp.async,
+// three rows ahead.  Per step, a lane keeps the populations that the rows below
+// will pull, already moved along x (one shuffle per population and row), the
+// pulled populations of the row it relaxes next, and psi of that row and the
+// one above with its neighbours' values (two shuffles per row): when input row
+// i has arrived, row i - 1 is pulled and its psi formed, and row i - 2 relaxed;
+// with two steps the relaxed row goes into a second such level at once and row
+// i - 4 goes to memory.  A step loses two columns on each side and two rows at
+// each end of an item: 56 of 64 columns are stored, and 4 (8) rows read beyond
+// an item's own.  Rows that do not start on 16 bytes are copied and stored per
+// node.  One warp per block: blocks refill as items end.
+//
+// Measured (GLUPS; in brackets the strips of 32 columns whose source rows
+// came through a per-warp shared-memory ring, one node per lane, which these
+// replace): 512 droplet domains of 64..512
+// 101 with two steps, 81 with one (72); 64 domains 88, 77 (66); 24 domains of
+// 64..128 31, 30 (9: one item per warp of an eight-warp block left most SMs
+// empty).  About 180 issue slots per 64 node updates, 347 per 32 for the row
+// ring.  Two steps move 40 B per node update and are bound by the latency of
+// their arithmetic chain at 12 warps per SM (168 registers), one step by
+// memory and the chain at 16.
 // ---------------------------------------------------------------------------
-constexpr int ENS_RING = 6;                    // source-row slots per warp
-constexpr int ENS_RCOLS = ET_BX + 8;           // columns x0 - 4 .. x0 + 35
-constexpr int ENS_RROW = 9 * ENS_RCOLS;        // floats per slot (90 chunks of 16 bytes)
-constexpr int ENS_RING_SMEM = ENS_RING * ENS_RROW * 4 * (ENS_MARCH_THREADS / 32);  // 69 120 B
+constexpr int EP_EDGE = 4, EP_COLS = 64 - 2 * EP_EDGE;
+constexpr int EP_RING = 4;
+constexpr int EP_ROW = 9 * 32;  // column pairs of a row's nine populations
+// resident blocks (warps) per SM by steps per launch
+constexpr int ep_blocks(int steps) { return steps == 1 ? 16 : 12; }
 
-__device__ __forceinline__ void ens_cp16(float *dst, const float *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
-                     (uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void ens_cp_commit() {
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-// this lane's commit groups except the newest N have landed
-template <int N>
-__device__ __forceinline__ void ens_cp_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+struct EnsPairArgs {
+    EnsArgs a;
+    int rows;  // rows of an item
+    PairConst c;
+};
+
+template <int BYTES> __device__ __forceinline__ void ep_copy(void *dst, const void *src) {
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(src)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(src)
+                     : "memory");
 }
 
-template <int R, int MINB, bool MOM>
-__global__ void __launch_bounds__(ENS_MARCH_THREADS, MINB) ens_ring_kernel(const EnsArgs a) {
-    constexpr unsigned FULL = 0xffffffffu;
-    extern __shared__ __align__(16) float ens_ring_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *const ring = ens_ring_smem + warp * ENS_RING * ENS_RROW;
-    const int warps_per_block = ENS_MARCH_THREADS / 32;
-    const int nwarps = gridDim.x * warps_per_block;
-    const bool edge = lane == 0 || lane == 31;
-    const int col = 4 + lane, hcol = lane == 0 ? 3 : 4 + ET_BX;  // ring columns of x, xh
-    for (int it = blockIdx.x * warps_per_block + warp; it < a.nitems; it += nwarps) {
-        const EnsItem dm = a.items[it];
-        if ((dm.W & 31) || (dm.off & 3)) continue;  // the work list gives this kernel none
-        const int y_end = min(dm.y + R, dm.H);
-        const bool small_h = dm.H < 4;
-        // this lane's chunks of a source row (chunk c = 10 k + q: population k,
-        // columns x0 - 4 + 4q .. + 3), addresses in row 0 of the domain
-        const float *cs[3];
+template <int STEPS, bool MOM>
+__global__ void __launch_bounds__(32, ep_blocks(STEPS))
+    ens_pair_kernel(const __grid_constant__ EnsPairArgs pa) {
+    const EnsArgs &a = pa.a;
+    const PairConst &c = pa.c;
+    extern __shared__ __align__(16) float2 ep_smem[];
+    const int lane = threadIdx.x;
+    const EnsItem dm = a.items[blockIdx.x];
+    const int W = dm.W, H = dm.H;
+    const int nr = min(pa.rows, H - dm.y);
+    const bool vec = ((W | dm.off) & 3) == 0;  // rows and tiles start on 16 bytes
+    const int ns = (W + EP_COLS - 1) / EP_COLS, tw = ((W + ns - 1) / ns + 3) & ~3;
+    const int nw = min(tw, W - dm.x);
+    const int xs = dm.x - EP_EDGE + 2 * lane;
+    int xa = xs % W;
+    xa += xa < 0 ? W : 0;
+    const int xb = xa == W - 1 ? 0 : xa + 1;
+    const bool own_a = xs >= dm.x && xs < dm.x + nw, own_b = xs + 1 >= dm.x && xs + 1 < dm.x + nw;
+    float2 *const ring = ep_smem + lane;
+    const int last = nr + 4 * STEPS;
+    int y = (dm.y - 2 * STEPS) % H;
+    y += y < 0 ? H : 0;
+    const float *cs[5];
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int c = min(lane + 32 * i, 89);
-            const int k = c / 10, q = c - 10 * k;
-            cs[i] = a.src[k] + dm.off + ens_wrap(dm.x - 4 + 4 * q, dm.W, false);
+    for (int j = 0; j < 5; j++) {
+        const int ch = min(lane + 32 * j, 143), k = ch >> 4;
+        cs[j] = a.src[0];
+#pragma unroll
+        for (int m = 1; m < 9; m++)
+            if (k == m) cs[j] = a.src[m];
+        int x = (dm.x - EP_EDGE + 4 * (ch & 15)) % W;
+        cs[j] += dm.off + (x < 0 ? x + W : x);
+    }
+    auto copy = [&](int i, int slot) {
+        if (i < last) {
+            float2 *const d = ring + slot * EP_ROW;
+            const uint32_t o = (uint32_t)y * (uint32_t)W;
+            if (vec) {
+#pragma unroll
+                for (int j = 0; j < 5; j++)
+                    if (lane + 32 * j < 144) ep_copy<16>(d - lane + 2 * (lane + 32 * j), cs[j] + o);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 9; k++) {
+                    ep_copy<4>(&d[k * 32].x, a.src[k] + dm.off + (o + xa));
+                    ep_copy<4>(&d[k * 32].y, a.src[k] + dm.off + (o + xb));
+                }
+            }
+            y = y == H - 1 ? 0 : y + 1;
         }
-        // source row sr of the item lives in slot (sr - (y - 2)) % ENS_RING
-        auto slot = [&](int i) { return ring + i * ENS_RROW; };
-        // source row sr into slot i as one commit group (empty past the item)
-        auto issue = [&](int sr, int i) {
-            if (sr <= y_end + 1) {
-                const long row = (long)dm.W * ens_wrap(sr, dm.H, small_h);
-                float *sl = slot(i);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    PairD2 d;
+    d.n0 = both(-a.w0); d.n1 = both(-a.w1); d.n5 = both(-a.w5);
+    d.mt = both(-dm.tau_inv);
+    const float2 tau = both(dm.tau_inv), mG = both(-dm.G), w1 = both(a.w1), w5 = both(a.w5);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll
-                for (int j = 0; j < 3; j++)
-                    if (lane + 32 * j < 90) ens_cp16(sl + 4 * (lane + 32 * j), cs[j] + row);
-            }
-            ens_cp_commit();
-        };
-        // pull of ring column cl of the row whose upstream rows (row - 1, row,
-        // row + 1) sit in slots im, i0, ip: population k from row - cr_k,
-        // column cl - cx_k
-        auto pull = [&](int cl, int im, int i0, int ip, float(&g)[9]) {
-            const float *sm = slot(im), *s0 = slot(i0), *sp = slot(ip);
+    for (int j = 0; j < EP_RING - 1; j++) copy(j, j);
+    // per level: populations 4, 7, 8 of the last row (p) and the one before it
+    // (q) and 0, 1, 3 of the last row (b), moved along x; the pulled populations
+    // and moments of the row that is relaxed next; psi (left, centre, right) of
+    // that row (s0) and of the one above it (sm)
+    float2 p[STEPS][3], q[STEPS][3], b[STEPS][3], G[STEPS][9], rho[STEPS], ux[STEPS], uy[STEPS];
+    float2 s0[STEPS][3], sm[STEPS][3];
 #pragma unroll
-            for (int k = 0; k < 9; k++) {
-                const float *sl = d2_cr(k) > 0 ? sm : (d2_cr(k) < 0 ? sp : s0);
-                g[k] = sl[k * ENS_RCOLS + cl - d2_cx(k)];
-            }
-        };
+    for (int t = 0; t < STEPS; t++) {
 #pragma unroll
-        for (int i = 0; i < ENS_RING; i++) issue(dm.y - 2 + i, i);  // source rows y - 2 .. y + 3
-        ens_cp_wait<ENS_RING - 4>();  // rows y - 2 .. y + 1 have landed
+        for (int j = 0; j < 3; j++)
+            p[t][j] = q[t][j] = b[t][j] = s0[t][j] = sm[t][j] = both(1.f);
+#pragma unroll
+        for (int k = 0; k < 9; k++) G[t][k] = both(1.f);
+        rho[t] = ux[t] = uy[t] = both(1.f);
+    }
+    int slot = 0, next = EP_RING - 1;
+#pragma unroll 1
+    for (int i = 0; i < last; i++) {
         __syncwarp();
-        float gc[9], rc, uxc, uyc;  // row r: pulled populations and moments at x
-        float pm, pc, hm = 0.f, hc = 0.f;  // psi of rows r - 1, r (h: the halo column)
-        {
-            float g[9];
-            pull(col, 0, 1, 2, g);
-            pm = ens_psi(a, d2q9_rho_native(g));
-            pull(col, 1, 2, 3, gc);
-            d2q9_moments_native(gc, rc, uxc, uyc);
-            pc = ens_psi(a, rc);
-            if (edge) {
-                pull(hcol, 0, 1, 2, g);
-                hm = ens_psi(a, d2q9_rho_native(g));
-                pull(hcol, 1, 2, 3, g);
-                hc = ens_psi(a, d2q9_rho_native(g));
-            }
-        }
-        auto next = [](int i) { return i == ENS_RING - 1 ? 0 : i + 1; };
-        int i0 = 2;  // slot of source row r
-        const int x = dm.x + lane;
-        for (int r = dm.y; r < y_end; r++) {
-            const int i1 = next(i0), i2 = next(i1);
-            __syncwarp();  // every lane is done with the slot of source row r - 2
-            issue(r + ENS_RING - 2, i0 >= 2 ? i0 - 2 : i0 + ENS_RING - 2);
-            ens_cp_wait<ENS_RING - 4>();  // source row r + 2 has landed
-            __syncwarp();
-            float gn[9], rn, uxn, uyn, hn = 0.f;
-            pull(col, i0, i1, i2, gn);
-            if (edge) {
-                float g[9];
-                pull(hcol, i0, i1, i2, g);
-                hn = ens_psi(a, d2q9_rho_native(g));
-            }
-            i0 = i1;
-            d2q9_moments_native(gn, rn, uxn, uyn);
-            const float pn = ens_psi(a, rn);
-            // x - 1 and x + 1 from the neighbour lanes, the halo at the strip ends
-            float lm = __shfl_up_sync(FULL, pm, 1), lc = __shfl_up_sync(FULL, pc, 1);
-            float ln = __shfl_up_sync(FULL, pn, 1);
-            float qm = __shfl_down_sync(FULL, pm, 1), qc = __shfl_down_sync(FULL, pc, 1);
-            float qn = __shfl_down_sync(FULL, pn, 1);
-            if (lane == 0) { lm = hm; lc = hc; ln = hn; }
-            if (lane == 31) { qm = hm; qc = hc; qn = hn; }
-            const float ps[9] = {pc, qc, pn, lc, pm, qn, ln, lm, qm};
-            float ex = uxc, ey = uyc;
-            d2q9_sc_shift_native(ps, a.w1, a.w5, dm.G, 1.f / (dm.tau_inv * rc), ex, ey);
-            d2q9_bgk_native(gc, ex, ey, rc, a.w0, a.w1, a.w5, dm.tau_inv);
-            const int o = dm.off + x + dm.W * r;
-            if (MOM) { a.rho[o] = rc; a.ux[o] = uxc; a.uy[o] = uyc; }
+        copy(i + EP_RING - 1, next);
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(EP_RING - 1) : "memory");
+        __syncwarp();
+        const float2 *const row = ring + slot * EP_ROW;
+        float2 n[9];
 #pragma unroll
-            for (int k = 0; k < 9; k++) a.dst[k][o] = gc[k];
+        for (int k = 0; k < 9; k++) n[k] = row[k * 32];
+        next = slot;
+        slot = slot == EP_RING - 1 ? 0 : slot + 1;
 #pragma unroll
-            for (int k = 0; k < 9; k++) gc[k] = gn[k];
-            rc = rn; uxc = uxn; uyc = uyn;
-            pm = pc; pc = pn; hm = hc; hc = hn;
+        for (int t = 0; t < STEPS; t++) {
+            // n: row j of the level below; pull row j - 1, relax row j - 2
+            float2 g[9];
+            g[0] = b[t][0]; g[1] = b[t][1]; g[3] = b[t][2];
+            g[4] = q[t][0]; g[7] = q[t][1]; g[8] = q[t][2];
+            g[2] = n[2];
+            g[5] = row_shift(n[5], d2_cx(5));
+            g[6] = row_shift(n[6], d2_cx(6));
+            b[t][0] = n[0];
+            b[t][1] = row_shift(n[1], d2_cx(1));
+            b[t][2] = row_shift(n[3], d2_cx(3));
+#pragma unroll
+            for (int j = 0; j < 3; j++) q[t][j] = p[t][j];
+            p[t][0] = n[4];
+            p[t][1] = row_shift(n[7], d2_cx(7));
+            p[t][2] = row_shift(n[8], d2_cx(8));
+            float2 r1, u1, v1;
+            d2q9_moments_pairs(c, g, r1, u1, v1);
+            const float2 ps = a.psi_form == 0 ? make_float2(psi_ref(r1.x), psi_ref(r1.y))
+                                              : pair_psi_exp1(c, r1);
+            const float2 sp[3] = {row_shift(ps, 1), ps, row_shift(ps, -1)};
+            // relax row j - 2: psi of the row above sm, its own s0, below sp
+            const float2 irt = pair_rcp(c, __fmul2_rn(tau, rho[t]));
+            const float2 ix = __ffma2_rn(
+                w1, pair_sub(c, s0[t][2], s0[t][0]),
+                __fmul2_rn(w5, pair_sub(c, pair_add(sp[2], sm[t][2]), pair_add(sp[0], sm[t][0]))));
+            const float2 iy = __ffma2_rn(
+                w1, pair_sub(c, sm[t][1], sp[1]),
+                __fmul2_rn(w5, pair_sub(c, pair_add(sm[t][0], sm[t][2]), pair_add(sp[2], sp[0]))));
+            const float2 cc = __fmul2_rn(__fmul2_rn(mG, s0[t][1]), irt);
+            const float2 ex = __ffma2_rn(cc, ix, ux[t]), ey = __ffma2_rn(cc, iy, uy[t]);
+            d2q9_bgk_pairs(c, d, G[t], ex, ey, rho[t]);
+            if (t < STEPS - 1) {
+#pragma unroll
+                for (int k = 0; k < 9; k++) n[k] = G[t][k];
+            } else if (i >= 4 * STEPS) {
+                const uint32_t o = (uint32_t)dm.off + (uint32_t)(dm.y + i - 4 * STEPS) * (uint32_t)W;
+                if (MOM) {
+                    if (own_a) { a.rho[o + xa] = rho[t].x; a.ux[o + xa] = ux[t].x; a.uy[o + xa] = uy[t].x; }
+                    if (own_b) { a.rho[o + xb] = rho[t].y; a.ux[o + xb] = ux[t].y; a.uy[o + xb] = uy[t].y; }
+                }
+                if (vec && own_a && own_b) {
+#pragma unroll
+                    for (int k = 0; k < 9; k++)
+                        *reinterpret_cast<float2 *>(a.dst[k] + (o + xa)) = G[t][k];
+                } else {
+                    if (own_a) {
+#pragma unroll
+                        for (int k = 0; k < 9; k++) a.dst[k][o + xa] = G[t][k].x;
+                    }
+                    if (own_b) {
+#pragma unroll
+                        for (int k = 0; k < 9; k++) a.dst[k][o + xb] = G[t][k].y;
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 9; k++) G[t][k] = g[k];
+            rho[t] = r1; ux[t] = u1; uy[t] = v1;
+#pragma unroll
+            for (int j = 0; j < 3; j++) { sm[t][j] = s0[t][j]; s0[t][j] = sp[j]; }
         }
-        __syncwarp();  // the next item's copies overwrite slots this item read
     }
-}
-
-// ring strip shapes: rows per item and the register bound (resident blocks per SM)
-#define LB_ENS_RING(X) \
-    X(10, 32, 3)       \
-    X(11, 64, 3)       \
-    X(12, 16, 3)
-
-int ens_ring_rows(int shape) {
-    switch (shape) {
-#define LB_ENS_RROWS(S, R, MINB) \
-    case S: return R;
-        LB_ENS_RING(LB_ENS_RROWS)
-#undef LB_ENS_RROWS
-        default: return 0;
-    }
-}
-
-template <int R, int MINB>
-cudaError_t ens_ring_launch(const EnsArgs &a, bool mom, unsigned grid, cudaStream_t s) {
-    // once per instantiation
-    static const cudaError_t attr_e[2] = {
-        cudaFuncSetAttribute(ens_ring_kernel<R, MINB, false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, ENS_RING_SMEM),
-        cudaFuncSetAttribute(ens_ring_kernel<R, MINB, true>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, ENS_RING_SMEM)};
-    if (attr_e[mom ? 1 : 0] != cudaSuccess) return attr_e[mom ? 1 : 0];
-    if (mom) ens_ring_kernel<R, MINB, true><<<grid, ENS_MARCH_THREADS, ENS_RING_SMEM, s>>>(a);
-    else ens_ring_kernel<R, MINB, false><<<grid, ENS_MARCH_THREADS, ENS_RING_SMEM, s>>>(a);
-    return cudaGetLastError();
 }
 
 // march shapes: rows per item and the register bound (resident blocks per SM)
@@ -515,10 +542,25 @@ int ens_tile_rows(int shape) {
 
 struct LaunchShape {
     int bx, ry, bps;  // threads along x, rows per work item (= blockDim.y), blocks per SM;
-                      // bx = 0: the single-pass tile kernel of tile shape ry
+                      // bx = 0: the single-pass form ry
 };
 
+// forms 10 to 12: the column-pair strips, by rows of an item (0: the library's
+// choice, and its choice of one or two steps per launch)
+bool ens_pairs(const LaunchShape &s) { return s.bx == 0 && s.ry >= 10 && s.ry <= 12; }
+int ens_pair_form_rows(int form) { return form == 11 ? 64 : form == 12 ? 16 : 0; }
+int ens_pair_tile(int W) {
+    const int ns = (W + EP_COLS - 1) / EP_COLS;
+    return ((W + ns - 1) / ns + 3) & ~3;
+}
+
 }  // namespace
+
+// Form 10 takes two steps per launch from this many nodes on (24 domains of 0.27
+// M nodes in all: 31.5 GLUPS with two, 30.2 with one; 64 of 6.6 M: 88 and 77) if
+// most of them lie in domains whose rows start on 16 bytes (400 domains of 97,
+// 101 and 130 columns: 39 GLUPS with two, 52 with one).
+constexpr long ENS_TWO_STEP_MIN_NODES = 1L << 20;
 
 struct lb_ensemble {
     int nd = 0;
@@ -528,12 +570,11 @@ struct lb_ensemble {
     float *psi = nullptr, *mom = nullptr;
     EnsItem *items_d = nullptr;
     int nitems = 0, items_cap = 0;
-    int nring = 0;  // ring strip shapes: the leading items the ring kernel takes
+    bool two_steps = false;  // form 10 advances two steps per launch
+    int pair_rows = 0;       // column-pair strips: rows of an item
     int cur = 0, psi_form = LB_PSI_EXP1, sms = 1, graph_steps = 32;
-    // single-pass warp strips of 32 rows with the shared-memory row ring, 3
-    // blocks per SM: 72.4 GLUPS on 512 droplet domains, against 63.2 for the
-    // strips with plain loads (shape 6)
-    LaunchShape shape{0, 10, 3};
+    // strips of column pairs
+    LaunchShape shape{0, 10, 12};
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -575,37 +616,37 @@ EnsArgs args_for(lb_ensemble *e, int from) {
 
 int launches_per_step(const lb_ensemble *e) {
     if (e->shape.bx != 0) return 2;
-    if (ens_ring_rows(e->shape.ry)) return (e->nring > 0) + (e->nitems > e->nring);
     return 1;
 }
 
-// ring strip shapes: the ring kernel over the leading qualifying items, the
-// plain march over the rest
-template <int R, int MINB>
-cudaError_t ens_ring_step(lb_ensemble *e, const EnsArgs &a, bool mom) {
-    const auto grid_for = [e](int n) {
-        return (unsigned)std::max(1, std::min(n, e->sms * e->shape.bps));
-    };
-    EnsArgs ar = a, am = a;
-    ar.nitems = e->nring;
-    am.items = a.items + e->nring;
-    am.nitems = a.nitems - e->nring;
-    if (ar.nitems > 0) {
-        const cudaError_t c = ens_ring_launch<R, MINB>(ar, mom, grid_for(ar.nitems), e->stream);
-        if (c != cudaSuccess) return c;
-        e->launches += 1;
-    }
-    if (am.nitems > 0) {
-        const unsigned g = grid_for(am.nitems);
-        if (mom) ens_march_kernel<R, MINB, true><<<g, ENS_MARCH_THREADS, 0, e->stream>>>(am);
-        else ens_march_kernel<R, MINB, false><<<g, ENS_MARCH_THREADS, 0, e->stream>>>(am);
-        e->launches += 1;
-        return cudaGetLastError();
-    }
-    return cudaSuccess;
+// column-pair strips: `steps` (1 or 2) steps in one launch, a programmatic
+// dependent of the launch before it
+cudaError_t ens_pair_launch(lb_ensemble *e, int from, int steps, bool mom) {
+    EnsPairArgs pa{};
+    pa.a = args_for(e, from);
+    pa.rows = e->pair_rows;
+    pa.c = pair_constants();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(e->nitems);
+    cfg.blockDim = dim3(32);
+    cfg.dynamicSmemBytes = EP_RING * EP_ROW * sizeof(float2);
+    cfg.stream = e->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e->launches += 1;
+    if (steps == 1)
+        return mom ? cudaLaunchKernelEx(&cfg, ens_pair_kernel<1, true>, pa)
+                   : cudaLaunchKernelEx(&cfg, ens_pair_kernel<1, false>, pa);
+    return mom ? cudaLaunchKernelEx(&cfg, ens_pair_kernel<2, true>, pa)
+               : cudaLaunchKernelEx(&cfg, ens_pair_kernel<2, false>, pa);
 }
 
+// one step (any form)
 cudaError_t ens_step(lb_ensemble *e, int from, bool mom) {
+    if (ens_pairs(e->shape)) return ens_pair_launch(e, from, 1, mom);
     const EnsArgs a = args_for(e, from);
     const unsigned grid = (unsigned)std::max(1, std::min(e->nitems, e->sms * e->shape.bps));
     if (e->shape.bx == 0) {
@@ -624,11 +665,6 @@ cudaError_t ens_step(lb_ensemble *e, int from, bool mom) {
         break;
             LB_ENS_MARCH(LB_ENS_MLAUNCH)
 #undef LB_ENS_MLAUNCH
-#define LB_ENS_RLAUNCH(S, R, MINB)                                                             \
-    case S:                                                                                    \
-        return ens_ring_step<R, MINB>(e, a, mom);
-            LB_ENS_RING(LB_ENS_RLAUNCH)
-#undef LB_ENS_RLAUNCH
             default: return cudaErrorInvalidValue;
         }
         e->launches += 1;
@@ -652,27 +688,66 @@ void drop_graphs(lb_ensemble *e) {
         }
 }
 
+// steps per launch of the current form, and such a launch
+int ens_steps_per_launch(const lb_ensemble *e) {
+    return e->shape.bx == 0 && e->shape.ry == 10 && e->two_steps ? 2 : 1;
+}
+cudaError_t ens_launch(lb_ensemble *e, int from, bool mom) {
+    const int s = ens_steps_per_launch(e);
+    return s > 1 ? ens_pair_launch(e, from, s, mom) : ens_step(e, from, mom);
+}
+
+// Column-pair strips: rows per item.  Fewer rows fill the GPU's warps, more rows
+// pay less for the 4 (8) rows an item reads beyond its own.  A pass takes an
+// item's march times a function of the rounds of items w that was fitted to 64
+// domains and two steps (us per step): 16 rows 89.7, 24 89.0, 32 88.3, 48 87.0,
+// 64 103 (w = 1.13: a nearly empty second round), 96 94.9 (w = 0.75).
+int ens_pick_rows(const lb_ensemble *e) {
+    const int steps = ens_steps_per_launch(e);
+    const double warps = (double)e->sms * ep_blocks(steps);
+    int pick = 8;
+    double best = 0;
+    for (int r : {8, 12, 16, 24, 32, 48, 64, 96, 128}) {
+        long items = 0;
+        for (const EnsDomain &m : e->dom) {
+            const int tw = ens_pair_tile(m.W);
+            items += (long)((m.W + tw - 1) / tw) * ((m.H + r - 1) / r);
+        }
+        const double w = items / warps;
+        const double cost = (r + 4. * steps) * (w <= 1. ? 0.65 + 0.35 * w : std::max(1.42, 0.32 + 0.82 * w));
+        if (best == 0 || cost < best) {
+            best = cost;
+            pick = r;
+        }
+    }
+    return pick;
+}
+
 // work list of row groups for the current shape
 int build_items(lb_ensemble *e) {
-    std::vector<EnsItem> items, rest;
+    std::vector<EnsItem> items;
+    const bool pairs = ens_pairs(e->shape);
+    if (pairs) {
+        const int r = ens_pair_form_rows(e->shape.ry);
+        e->pair_rows = r ? r : ens_pick_rows(e);
+    }
     for (int d = 0; d < e->nd; d++) {
         const EnsDomain &m = e->dom[d];
-        if (e->shape.bx == 0) {  // tiles or strips, row by row
-            const int rows = ens_tile_rows(e->shape.ry) + ens_march_rows(e->shape.ry) +
-                             ens_ring_rows(e->shape.ry);
-            // ring strips: the items the ring kernel takes first, the rest after
-            const bool ring = ens_ring_rows(e->shape.ry) > 0;
-            std::vector<EnsItem> &to = ring && ((m.W & 31) || (m.off & 3)) ? rest : items;
+        if (pairs) {
+            const int tw = ens_pair_tile(m.W);
+            for (int y = 0; y < m.H; y += e->pair_rows)
+                for (int x = 0; x < m.W; x += tw)
+                    items.push_back(EnsItem{m.off, m.W, m.H, y, m.G, m.tau_inv, x});
+        } else if (e->shape.bx == 0) {  // tiles or strips, row by row
+            const int rows = ens_tile_rows(e->shape.ry) + ens_march_rows(e->shape.ry);
             for (int y = 0; y < m.H; y += rows)
                 for (int x = 0; x < m.W; x += ET_BX)
-                    to.push_back(EnsItem{m.off, m.W, m.H, y, m.G, m.tau_inv, x});
+                    items.push_back(EnsItem{m.off, m.W, m.H, y, m.G, m.tau_inv, x});
         } else {  // groups of ry rows
             for (int y = 0; y < m.H; y += e->shape.ry)
                 items.push_back(EnsItem{m.off, m.W, m.H, y, m.G, m.tau_inv, 0});
         }
     }
-    e->nring = (int)items.size();
-    items.insert(items.end(), rest.begin(), rest.end());
     if ((int)items.size() > e->items_cap) {
         if (e->items_d) cudaFree(e->items_d);
         e->items_d = nullptr;
@@ -692,8 +767,9 @@ int egraph(lb_ensemble *e, int from, cudaGraphExec_t *out) {
     LB_ETRY(e, "capture", cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t c = cudaSuccess;
     int set = from;
-    for (int i = 0; i < e->graph_steps && c == cudaSuccess; i++) {
-        c = ens_step(e, set, false);
+    const int launches = e->graph_steps / ens_steps_per_launch(e);  // even: back to `from`
+    for (int i = 0; i < launches && c == cudaSuccess; i++) {
+        c = ens_launch(e, set, false);
         set = 1 - set;
     }
     cudaGraph_t g;
@@ -729,6 +805,10 @@ int lb_ensemble_create(int nd, const int *nx, const int *ny, const float *G, con
     }
     e->NT = off;
     e->stride = (off + 127) / 128 * 128;
+    long aligned = 0;
+    for (const EnsDomain &m : e->dom)
+        if (((m.W | m.off) & 3) == 0) aligned += (long)m.W * m.H;
+    e->two_steps = off >= ENS_TWO_STEP_MIN_NODES && 2 * aligned >= off;
     int dev = 0;
     cudaError_t c = cudaGetDevice(&dev);
     if (c == cudaSuccess) c = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, dev);
@@ -745,6 +825,18 @@ int lb_ensemble_create(int nd, const int *nx, const int *ny, const float *G, con
         return c == cudaErrorMemoryAllocation ? LB_ERR_NOMEM : LB_ERR_CUDA;
     }
     if (build_items(e) != LB_OK) {
+        lb_ensemble_destroy(e);
+        return LB_ERR_CUDA;
+    }
+    // at rest at density 1 until the caller sets a state: the autotuner, which
+    // runs before that, would otherwise time the steps on whatever the memory
+    // holds (divisions by zero, not numbers)
+    Pop<9> p;
+    for (int k = 0; k < 9; k++) p.f[k] = pk(e, e->cur, k);
+    c = launch_d2q9_equilibrium(p, nullptr, nullptr, nullptr, (int)e->NT, W2F[0], W2F[1], W2F[2],
+                                e->stream);
+    if (c == cudaSuccess) c = cudaStreamSynchronize(e->stream);
+    if (c != cudaSuccess) {
         lb_ensemble_destroy(e);
         return LB_ERR_CUDA;
     }
@@ -812,21 +904,24 @@ int lb_ensemble_init_equilibrium(lb_ensemble *e, const float *rho) {
 int lb_ensemble_step(lb_ensemble *e, int nsteps) {
     if (!e || nsteps < 0) return LB_ERR_ARG;
     if (nsteps == 0) return LB_OK;
-    int rest = nsteps - 1;
-    while (rest >= e->graph_steps) {
+    const int per = ens_steps_per_launch(e);
+    int rest = nsteps;
+    for (; rest % per; rest--) {  // single steps first: the last launch writes the moments
+        LB_ETRY(e, "lb_ensemble_step", ens_step(e, e->cur, rest == 1));
+        e->cur = 1 - e->cur;
+    }
+    while (rest > e->graph_steps) {
         cudaGraphExec_t g;
         const int rc = egraph(e, e->cur, &g);
         if (rc != LB_OK) return rc;
         LB_ETRY(e, "cudaGraphLaunch", cudaGraphLaunch(g, e->stream));
-        e->launches += (int64_t)launches_per_step(e) * e->graph_steps;
+        e->launches += (int64_t)launches_per_step(e) * (e->graph_steps / per);
         rest -= e->graph_steps;
     }
-    for (; rest > 0; rest--) {
-        LB_ETRY(e, "lb_ensemble_step", ens_step(e, e->cur, false));
+    for (; rest > 0; rest -= per) {
+        LB_ETRY(e, "lb_ensemble_step", ens_launch(e, e->cur, rest == per));
         e->cur = 1 - e->cur;
     }
-    LB_ETRY(e, "lb_ensemble_step", ens_step(e, e->cur, true));
-    e->cur = 1 - e->cur;
     return LB_OK;
 }
 
@@ -856,7 +951,8 @@ int lb_ensemble_get_moments(lb_ensemble *e, float *rho, float *ux, float *uy) {
 int lb_ensemble_set_launch(lb_ensemble *e, int threads_x, int rows, int blocks_per_sm) {
     const bool tiles = threads_x == 0;
     if (!e || blocks_per_sm < 1 || blocks_per_sm > 32 ||
-        (tiles && ens_tile_rows(rows) + ens_march_rows(rows) + ens_ring_rows(rows) == 0) ||
+        (tiles && ens_tile_rows(rows) + ens_march_rows(rows) == 0 &&
+         !ens_pairs(LaunchShape{0, rows, 1})) ||
         (!tiles && (threads_x < 32 || threads_x % 32 || rows < 1 || threads_x * rows > 1024)))
         return LB_ERR_ARG;
     LB_ETRY(e, "lb_ensemble_set_launch", cudaStreamSynchronize(e->stream));
@@ -883,7 +979,7 @@ int lb_ensemble_autotune(lb_ensemble *e, int trial_steps, int out[3]) {
     // residency and at twice it
     static const int TILES[][2] = {{1, 5}, {1, 10}, {2, 6}, {2, 12}, {3, 2}, {3, 4}, {4, 3},
                                    {5, 1}, {6, 3}, {6, 6}, {7, 4}, {7, 8}, {8, 3}, {9, 3},
-                                   {10, 3}, {11, 3}, {12, 3}};
+                                   {10, 12}, {11, 12}, {12, 12}};
     std::vector<LaunchShape> cand;
     for (const auto &t : TILES) cand.push_back(LaunchShape{0, t[0], t[1]});
     for (int i = 0; i < 3; i++)
@@ -895,17 +991,19 @@ int lb_ensemble_autotune(lb_ensemble *e, int trial_steps, int out[3]) {
     for (const LaunchShape &c : cand) {
         int rc = lb_ensemble_set_launch(e, c.bx, c.ry, c.bps);
         if (rc != LB_OK) return rc;
-        LB_ETRY(e, "autotune", ens_step(e, e->cur, false));  // one untimed step
+        LB_ETRY(e, "autotune", ens_launch(e, e->cur, false));  // one untimed launch
         e->cur = 1 - e->cur;
+        const int per = ens_steps_per_launch(e), trials = (trial_steps + per - 1) / per;
         LB_ETRY(e, "autotune", cudaEventRecord(e->ev0, e->stream));
-        for (int s = 0; s < trial_steps; s++) {
-            LB_ETRY(e, "autotune", ens_step(e, e->cur, false));
+        for (int s = 0; s < trials; s++) {
+            LB_ETRY(e, "autotune", ens_launch(e, e->cur, false));
             e->cur = 1 - e->cur;
         }
         LB_ETRY(e, "autotune", cudaEventRecord(e->ev1, e->stream));
         LB_ETRY(e, "autotune", cudaEventSynchronize(e->ev1));
         float ms = 0.f;
         LB_ETRY(e, "autotune", cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+        ms /= trials * per;  // a step
         if (ms < best) {
             best = ms;
             pick = e->shape;

@@ -57,9 +57,33 @@ struct PairD2 {
     float2 n0, n1, n5, mt, tau, Fx, Fy;
 };
 
-// d2q9_collide_native of two nodes (force: Fx or Fy is not zero)
-__device__ __forceinline__ void d2q9_collide_pairs(const PairConst &c, const PairD2 &d,
-                                                   float2 (&g)[9], bool force,
+// psi = 1 - exp(-rho) of both lanes: psi_exp1's operations (lb_expf for |x| <= 87,
+// the scalar form beyond; the first product of its reduction is exact, so its
+// subtraction may be fused)
+__device__ __forceinline__ float2 pair_psi_exp1(const PairConst &c, float2 rho) {
+    const float2 x = __fmul2_rn(rho, c.mone);
+    const float2 s = __ffma2_rn(__fmul2_rn(x, both(0x1.715476p+0f)), c.one, both(0x1.8p+23f));
+    const float2 k = pair_add(s, both(-0x1.8p+23f));
+    const float2 d = __ffma2_rn(k, both(-0x1.62ep-1f), x);
+    const float2 r = __ffma2_rn(__fmul2_rn(k, both(0x1.0bfbe8p-15f)), c.mone, d);
+    float2 p = both(0x1.a01a02p-13f);
+    const auto horner = [&](float a) { p = __ffma2_rn(__fmul2_rn(p, r), c.one, both(a)); };
+    horner(0x1.6c16c2p-10f);
+    horner(0x1.111112p-7f);
+    horner(0x1.555556p-5f);
+    horner(0x1.555556p-3f);
+    horner(0.5f);
+    horner(1.0f);
+    horner(1.0f);
+    const float2 two_k = make_float2(__int_as_float((__float_as_int(s.x) << 23) + 0x3f800000),
+                                     __int_as_float((__float_as_int(s.y) << 23) + 0x3f800000));
+    const float2 psi = __ffma2_rn(__fmul2_rn(p, two_k), c.mone, c.one);
+    if (fabsf(x.x) <= 87.f && fabsf(x.y) <= 87.f) return psi;
+    return make_float2(psi_exp1(rho.x), psi_exp1(rho.y));
+}
+
+// d2q9_moments_native of two nodes
+__device__ __forceinline__ void d2q9_moments_pairs(const PairConst &c, const float2 (&g)[9],
                                                    float2 &rho, float2 &ux, float2 &uy) {
     const auto add = [](float2 a, float2 b) { return pair_add(a, b); };
     const float2 px = add(add(g[1], g[5]), g[8]);
@@ -70,12 +94,11 @@ __device__ __forceinline__ void d2q9_collide_pairs(const PairConst &c, const Pai
     const float2 inv = pair_rcp(c, rho);
     ux = __fmul2_rn(pair_sub(c, px, mx), inv);
     uy = __fmul2_rn(jy, inv);
-    float2 ex = ux, ey = uy;
-    if (force) {
-        const float2 irt = pair_rcp(c, __fmul2_rn(rho, d.tau));
-        if (d.Fx.x != 0.f) ex = __ffma2_rn(d.Fx, irt, ux);
-        if (d.Fy.x != 0.f) ey = __ffma2_rn(d.Fy, irt, uy);
-    }
+}
+
+// d2q9_bgk_native of two nodes
+__device__ __forceinline__ void d2q9_bgk_pairs(const PairConst &c, const PairD2 &d,
+                                               float2 (&g)[9], float2 ex, float2 ey, float2 rho) {
     const float2 usq = __ffma2_rn(ey, ey, __fmul2_rn(ex, ex));
     const float2 base = __ffma2_rn(c.m15, usq, c.one);
     // e = -(f_eq - g) in one rounding, then g - tau_inv e: the scalar form with
@@ -92,6 +115,20 @@ __device__ __forceinline__ void d2q9_collide_pairs(const PairConst &c, const Pai
     pair(2, 4, n1, ey);
     pair(5, 7, n5, pair_addp(c, ex, ey));
     pair(6, 8, n5, pair_sub(c, ey, ex));
+}
+
+// d2q9_collide_native of two nodes (force: Fx or Fy is not zero)
+__device__ __forceinline__ void d2q9_collide_pairs(const PairConst &c, const PairD2 &d,
+                                                   float2 (&g)[9], bool force, float2 &rho,
+                                                   float2 &ux, float2 &uy) {
+    d2q9_moments_pairs(c, g, rho, ux, uy);
+    float2 ex = ux, ey = uy;
+    if (force) {
+        const float2 irt = pair_rcp(c, __fmul2_rn(rho, d.tau));
+        if (d.Fx.x != 0.f) ex = __ffma2_rn(d.Fx, irt, ux);
+        if (d.Fy.x != 0.f) ey = __ffma2_rn(d.Fy, irt, uy);
+    }
+    d2q9_bgk_pairs(c, d, g, ex, ey, rho);
 }
 
 // a row's column pairs (lane l: columns 2l, 2l + 1) read one column to the left
