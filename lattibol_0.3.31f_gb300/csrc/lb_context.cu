@@ -60,10 +60,6 @@ struct lb_ctx {
     bool interior_pending = false;       // `side` holds interior planes `stream` has not joined
     void *face[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // group exchange [parity][below/above]
     int parity = 0;
-    // staged Shan-Chen step: tensor maps of the two population sets (TMA
-    // copies of the interior tiles' stages); 0 unknown, 1 encoded, -1 not available
-    CUtensorMap tmap[2];
-    int tmap_state[2] = {0, 0};
     // lb_slab_group_step on this slab as the group's first: graph-captured
     // batches of steps of the group (key: the group's slab list), one graph
     // per starting (population set, face parity)
@@ -100,10 +96,8 @@ int cuda_fail(lb_ctx *c, const char *where, cudaError_t e) {
 // stays (900^2: 99, the strips 115; 720^2: 97 and 90): there the strips have
 // too few warps to gain much, and a 1024^2 lattice is held to one launch per
 // step by its launch count.  D3Q19 Shan-Chen without walls: the
-// staged single-pass step measured 28.6 / 34.1 / 34.2 GLUPS (FP32 / FP16 /
-// BF16) at 256^3 against 26.4 / 31.5 / 31.5 for the density pass + fused step
-// (34.9 / 40.3 / 40.4 with compact stages, two steps per loop iteration, 3
-// blocks per SM and 32-bit chunk offsets).
+// staged single-pass step measures 35.9 / 53.9 / 54.1 GLUPS (FP32 / FP16 /
+// BF16) at 256^3 against 26.4 / 31.5 / 31.5 for the density pass + fused step.
 constexpr int LB_TUNE_LIBRARY_DEFAULT_D3 = LB_TUNE_REVERSE | LB_TUNE_SC_STAGED;
 constexpr int LB_TUNE_LIBRARY_DEFAULT_D2 = LB_TUNE_PDL;
 constexpr int TBLOCK_DEFAULT_SHAPE = 5;
@@ -163,7 +157,7 @@ bool sc_stage_on(const lb_ctx *c) {
     // (the kernel addresses the populations as 32-bit element offsets from the
     // first array: all 19 must lie within 2^32 elements of it)
     return c->Q == 19 && c->cfg.mode == LB_MODE_NATIVE && sc_on(c) && !c->any_wall &&
-           (c->tune & LB_TUNE_SC_STAGED) && sc_stage_chunk(c->cfg.nx, c->cfg.ny, c->cfg.nz) &&
+           (c->tune & LB_TUNE_SC_STAGED) && sc_stage_fits(c->cfg.nx, c->cfg.ny, c->cfg.nz) &&
            19L * c->stride < (1L << 32);
 }
 
@@ -312,16 +306,7 @@ cudaError_t step_once(lb_ctx *c, int from, bool moments) {
             c->launches += 1;
             a.err = c->errw;
             c->err_pending = true;  // a block that gave up waiting reports through the error word
-            // TMA copies for the 16-bit storage forms (42.0 vs 39.3 GLUPS at 256^3
-            // against the same layout by cp.async); FP32 keeps the compact
-            // cp.async stages (TMA measured 27.1 against 32.6 and 34.9 compact)
-            if (!c->tmap_state[from])
-                c->tmap_state[from] =
-                    (c->tune & LB_TUNE_SC_NO_TMA) || g.storage == LB_STORE_F32 ? -1
-                    : sc_stage_tensor_map(a, g.storage, &c->tmap[from]) ? 1 : -1;
-            return launch_d3q19_sc_stage(a, g.storage, moments,
-                                         c->tmap_state[from] > 0 ? &c->tmap[from] : nullptr,
-                                         c->stream);
+            return launch_d3q19_sc_stage(a, g.storage, moments, c->stream);
         }
         c->launches += sc ? 2 : 1;
         return launch_d3q19_native(a, g.storage, moments, sc, c->stream);

@@ -3,7 +3,6 @@
 // (lb_abi.cu, lb_context.cu).
 #pragma once
 
-#include <cuda.h>
 
 #include "lb_common.cuh"
 #include "lb_mlp.cuh"
@@ -111,16 +110,10 @@ cudaError_t launch_plane_copy(const void *const *src, void *const *dst, int n, l
                               cudaStream_t s);
 // single-pass Shan-Chen step whose populations arrive by bulk asynchronous
 // copies (lb_sc_stage.cu); lattices without wall nodes for which
-// sc_stage_chunk(W, H, D) != 0.  A block that gives up waiting for its copies
+// sc_stage_fits.  A block that gives up waiting for its copies
 // sets *a.err (when a.err is set).
-int sc_stage_chunk(int W, int H, int D);
-// tmap: the tensor map of a.src (sc_stage_tensor_map) for the blocks whose
-// stages lie inside the lattice, or null (every stage by cp.async chunks)
-cudaError_t launch_d3q19_sc_stage(const D3Args &a, int storage, bool mom,
-                                  const CUtensorMap *tmap, cudaStream_t s);
-// the tensor map the staged step reads a.src through; false if it cannot be
-// encoded (no driver entry point, or a layout it does not describe)
-bool sc_stage_tensor_map(const D3Args &a, int storage, CUtensorMap *out);
+bool sc_stage_fits(int W, int H, int D);
+cudaError_t launch_d3q19_sc_stage(const D3Args &a, int storage, bool mom, cudaStream_t s);
 // self-check of the staged step's bounded wait: one block whose first stage
 // waits get no polls gives up, sets *err (device memory) and returns
 cudaError_t sc_stage_wait_selftest(int *err);

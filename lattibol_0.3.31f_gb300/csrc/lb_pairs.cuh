@@ -52,6 +52,24 @@ __device__ __forceinline__ float2 pair_rcp(const PairConst &c, float2 x) {
     return make_float2(1.f / x.x, 1.f / x.y);
 }
 
+// two reciprocals at once (a check for both)
+__device__ __forceinline__ void pair_rcp2(const PairConst &c, float2 &x, float2 &y) {
+    float2 p, q;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(p.x) : "f"(x.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(p.y) : "f"(x.y));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q.x) : "f"(y.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q.y) : "f"(y.y));
+    const float2 e = __ffma2_rn(__fmul2_rn(x, c.mone), p, c.one);
+    const float2 f = __ffma2_rn(__fmul2_rn(y, c.mone), q, c.one);
+    if ((fabsf(e.x) + fabsf(e.y)) + (fabsf(f.x) + fabsf(f.y)) < 0.5f) {
+        x = __ffma2_rn(p, e, p);
+        y = __ffma2_rn(q, f, q);
+        return;
+    }
+    x = make_float2(1.f / x.x, 1.f / x.y);
+    y = make_float2(1.f / y.x, 1.f / y.y);
+}
+
 // the step's physics in paired form: -w0, -w1, -w5, -tau_inv, tau_inv, force
 struct PairD2 {
     float2 n0, n1, n5, mt, tau, Fx, Fy;
