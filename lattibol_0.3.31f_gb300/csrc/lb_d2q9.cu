@@ -35,10 +35,7 @@ struct Nbr2 {
 // which also makes that step's stores visible) before touching memory.
 template <int MODE, bool MOM, bool PLOT, bool SC, bool PDL = false>
 __global__ void __launch_bounds__(D2_BLOCK) d2q9_fused_kernel(const D2Args a) {
-    if (PDL) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    }
+    if (PDL) after_predecessor();
     const int bx = a.reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     const int x = bx * blockDim.x + threadIdx.x;
     const int y = a.reverse ? a.H - 1 - (int)blockIdx.y : (int)blockIdx.y;
@@ -165,6 +162,7 @@ __device__ __forceinline__ void d2q9_adhesion_sums(const uint8_t *s, int m1, int
 
 template <int MODE, bool PLOT>
 __global__ void __launch_bounds__(D2_BLOCK) d2q9_sc_kernel(const D2Args a) {
+    after_predecessor();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= a.W) return;
@@ -223,6 +221,7 @@ __global__ void __launch_bounds__(D2_BLOCK) d2q9_sc_kernel(const D2Args a) {
 // Reference-exact standalone streaming, src/streaming.cu:24-74.
 __global__ void __launch_bounds__(D2_BLOCK) d2q9_stream_swap_kernel(Pop<9> p, const uint8_t *sb,
                                                                    int W, int H) {
+    after_predecessor();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= W) return;
@@ -243,6 +242,7 @@ __global__ void __launch_bounds__(D2_BLOCK) d2q9_stream_swap_kernel(Pop<9> p, co
 // (the Shan-Chen pass is d2q9_sc_kernel, launched after it when G < 0).
 template <bool PLOT>
 __global__ void __launch_bounds__(D2_BLOCK) d2q9_collide_kernel(const D2Args a) {
+    after_predecessor();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= a.W) return;
@@ -318,10 +318,12 @@ cudaError_t launch_d2q9_fused(const D2Args &a0, int mode, bool mom, bool plot, c
     if (sc) mom = true;  // the second pass reads rho
 #define LB_D2_CASE(M, MO, PL, SC)                                                 \
     if (mode == M && mom == MO && plot == PL && sc == SC) {                       \
-        d2q9_fused_kernel<M, MO, PL, SC><<<g, b, 0, s>>>(a);                     \
+        e = PL || SC ? launch_dependent(d2q9_fused_kernel<M, MO, PL, SC, true>, g, b, s, a) \
+                     : (d2q9_fused_kernel<M, MO, PL, SC><<<g, b, 0, s>>>(a), cudaGetLastError()); \
         ok = true;                                                                \
     }
     bool ok = false;
+    cudaError_t e = cudaSuccess;
     LB_D2_CASE(MODE_REF, true, true, false)
     LB_D2_CASE(MODE_REF, true, false, false)
     LB_D2_CASE(MODE_REF, false, false, false)
@@ -334,53 +336,40 @@ cudaError_t launch_d2q9_fused(const D2Args &a0, int mode, bool mom, bool plot, c
     LB_D2_CASE(MODE_NATIVE, true, true, true)
 #undef LB_D2_CASE
     if (!ok) return cudaErrorInvalidValue;
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !sc_pass) return e;
-    if (mode == MODE_REF) {
-        if (plot) d2q9_sc_kernel<MODE_REF, true><<<g, b, 0, s>>>(a);
-        else d2q9_sc_kernel<MODE_REF, false><<<g, b, 0, s>>>(a);
-    } else {
-        if (plot) d2q9_sc_kernel<MODE_NATIVE, true><<<g, b, 0, s>>>(a);
-        else d2q9_sc_kernel<MODE_NATIVE, false><<<g, b, 0, s>>>(a);
-    }
-    return cudaGetLastError();
+    if (mode == MODE_REF)
+        return launch_dependent(plot ? d2q9_sc_kernel<MODE_REF, true>
+                                     : d2q9_sc_kernel<MODE_REF, false>, g, b, s, a);
+    return launch_dependent(plot ? d2q9_sc_kernel<MODE_NATIVE, true>
+                                 : d2q9_sc_kernel<MODE_NATIVE, false>, g, b, s, a);
 }
 
 cudaError_t launch_d2q9_fused_pdl(const D2Args &a0, int mode, bool mom, cudaStream_t s) {
     const D2Args a = with_zou_he(a0);
     if (a.G != 0.f) return cudaErrorInvalidValue;  // no Shan-Chen pass here
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid2(a.W, a.H);
-    cfg.blockDim = dim3(D2_BLOCK);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    const dim3 g = grid2(a.W, a.H), b(D2_BLOCK);
     if (mode == MODE_REF)
-        return mom ? cudaLaunchKernelEx(&cfg, d2q9_fused_kernel<MODE_REF, true, false, false, true>, a)
-                   : cudaLaunchKernelEx(&cfg, d2q9_fused_kernel<MODE_REF, false, false, false, true>, a);
-    return mom ? cudaLaunchKernelEx(&cfg, d2q9_fused_kernel<MODE_NATIVE, true, false, false, true>, a)
-               : cudaLaunchKernelEx(&cfg, d2q9_fused_kernel<MODE_NATIVE, false, false, false, true>, a);
+        return launch_dependent(mom ? d2q9_fused_kernel<MODE_REF, true, false, false, true>
+                                    : d2q9_fused_kernel<MODE_REF, false, false, false, true>,
+                                g, b, s, a);
+    return launch_dependent(mom ? d2q9_fused_kernel<MODE_NATIVE, true, false, false, true>
+                                : d2q9_fused_kernel<MODE_NATIVE, false, false, false, true>,
+                            g, b, s, a);
 }
 
 cudaError_t launch_d2q9_stream_swap(const Pop<9> &p, const uint8_t *sb, int W, int H,
                                     cudaStream_t s) {
-    d2q9_stream_swap_kernel<<<grid2(W, H), D2_BLOCK, 0, s>>>(p, sb, W, H);
-    return cudaGetLastError();
+    return launch_dependent(d2q9_stream_swap_kernel, grid2(W, H), dim3(D2_BLOCK), s, p, sb, W, H);
 }
 
 cudaError_t launch_d2q9_collide(const D2Args &a0, bool plot, cudaStream_t s) {
     const D2Args a = with_zou_he(a0);
     const dim3 g = grid2(a.W, a.H), b(D2_BLOCK);
-    if (plot) d2q9_collide_kernel<true><<<g, b, 0, s>>>(a);
-    else d2q9_collide_kernel<false><<<g, b, 0, s>>>(a);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_dependent(plot ? d2q9_collide_kernel<true>
+                                                : d2q9_collide_kernel<false>, g, b, s, a);
     if (e != cudaSuccess || !(a.G < 0.f)) return e;
-    if (plot) d2q9_sc_kernel<MODE_REF, true><<<g, b, 0, s>>>(a);
-    else d2q9_sc_kernel<MODE_REF, false><<<g, b, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(plot ? d2q9_sc_kernel<MODE_REF, true>
+                                 : d2q9_sc_kernel<MODE_REF, false>, g, b, s, a);
 }
 
 cudaError_t launch_d2q9_get_border(const CPop<9> &p, const Pop<6> &b, int W, int H,

@@ -95,6 +95,30 @@ template <typename Args> Args with_zou_he(const Args &a0) {
     return a;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may
+// start while the launch before it in the stream drains; its first statement,
+// after_predecessor(), waits for that launch's completion (and so for all
+// before it, which did the same or were complete when it started) and lets the
+// next one start.
+__device__ __forceinline__ void after_predecessor() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s,
+                             const A &...args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // D3Q19
 cudaError_t launch_d3q19_fused(const D3Args &a, int mode, bool mom, bool plot, cudaStream_t s);
 // native mode with storage kind (0 f32, 1 f16, 2 bf16) and optional Shan-Chen

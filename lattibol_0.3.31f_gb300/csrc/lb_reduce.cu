@@ -17,6 +17,7 @@ int reduce_partials_size() { return RED_BLOCKS * RED_FIELDS; }
 // plot buffer the probe reads the moment arrays
 __global__ void read_value_kernel(const float4 *plot, const float *ux, const float *uy,
                                   const float *uz, const float *rho, float *value, long o) {
+    after_predecessor();
     if (plot) {
         const float4 v = plot[o];
         value[0] = v.x; value[1] = v.y; value[2] = v.z; value[3] = v.w;
@@ -28,9 +29,8 @@ __global__ void read_value_kernel(const float4 *plot, const float *ux, const flo
 cudaError_t launch_read_value(const float *plot, const float *ux, const float *uy,
                              const float *uz, const float *rho, float *value, long o,
                              cudaStream_t s) {
-    read_value_kernel<<<1, 32, 0, s>>>(reinterpret_cast<const float4 *>(plot), ux, uy, uz, rho,
-                                       value, o);
-    return cudaGetLastError();
+    return launch_dependent(read_value_kernel, dim3(1), dim3(32), s,
+                            reinterpret_cast<const float4 *>(plot), ux, uy, uz, rho, value, o);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
