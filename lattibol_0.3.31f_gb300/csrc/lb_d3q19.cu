@@ -46,6 +46,7 @@ static_assert(D3_BLOCK * 2 == 256, "two 128-byte lines per 16-bit population run
 template <int MODE, bool MOM, bool PLOT, typename S, bool SC>
 __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
     d3q19_fused_kernel(const D3Args a) {
+    after_predecessor();
     const Coord3 c(a);
     const int x = c.x, y = c.y, z = c.z;
     if (x >= a.W) return;
@@ -143,6 +144,7 @@ __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
 // fused kernel computes), 0 at walls.
 template <typename S>
 __global__ void __launch_bounds__(D3_BLOCK) d3q19_density_kernel(const D3Args a) {
+    after_predecessor();
     const Coord3 c(a);
     if (c.x >= a.W) return;
     const int o = c.x + a.W * (c.y + a.H * c.z);
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(D3_BLOCK) d3q19_density_kernel(const D3Args a)
 __global__ void __launch_bounds__(D3_BLOCK) d3q19_stream_swap_kernel(Pop<19> p,
                                                                     const uint8_t *sb, int W,
                                                                     int H, int D) {
+    after_predecessor();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y, z = blockIdx.z;
     if (x >= W) return;
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(D3_BLOCK) d3q19_stream_swap_kernel(Pop<19> p,
 // Reference-exact standalone collision, src/collision.cu:357-552.
 template <bool PLOT>
 __global__ void __launch_bounds__(D3_BLOCK) d3q19_collide_kernel(const D3Args a) {
+    after_predecessor();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y, z = blockIdx.z;
     if (x >= a.W) return;
@@ -311,8 +315,7 @@ cudaError_t launch_d3q19_fused(const D3Args &a0, int mode, bool mom, bool plot, 
     const dim3 g = grid_of(a.W, a.H, a.D), b(D3_BLOCK);
 #define LB_D3_CASE(M, MO, PL)                                                    \
     if (mode == M && mom == MO && plot == PL) {                                  \
-        d3q19_fused_kernel<M, MO, PL, float, false><<<g, b, 0, s>>>(a);         \
-        return cudaGetLastError();                                               \
+        return launch_dependent(d3q19_fused_kernel<M, MO, PL, float, false>, g, b, s, a); \
     }
     LB_D3_CASE(MODE_REF, true, true)
     LB_D3_CASE(MODE_REF, true, false)
@@ -327,16 +330,15 @@ template <typename S>
 static cudaError_t native_launch(const D3Args &a, bool mom, bool sc, cudaStream_t s) {
     const dim3 g = grid_of(a.W, a.H, a.D), b(D3_BLOCK);
     if (sc) {
-        d3q19_density_kernel<S><<<g, b, 0, s>>>(a);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_dependent(d3q19_density_kernel<S>, g, b, s, a);
         if (e != cudaSuccess) return e;
-        if (mom) d3q19_fused_kernel<MODE_NATIVE, true, false, S, true><<<g, b, 0, s>>>(a);
-        else d3q19_fused_kernel<MODE_NATIVE, false, false, S, true><<<g, b, 0, s>>>(a);
-    } else {
-        if (mom) d3q19_fused_kernel<MODE_NATIVE, true, false, S, false><<<g, b, 0, s>>>(a);
-        else d3q19_fused_kernel<MODE_NATIVE, false, false, S, false><<<g, b, 0, s>>>(a);
+        return launch_dependent(mom ? d3q19_fused_kernel<MODE_NATIVE, true, false, S, true>
+                                    : d3q19_fused_kernel<MODE_NATIVE, false, false, S, true>,
+                                g, b, s, a);
     }
-    return cudaGetLastError();
+    return launch_dependent(mom ? d3q19_fused_kernel<MODE_NATIVE, true, false, S, false>
+                                : d3q19_fused_kernel<MODE_NATIVE, false, false, S, false>,
+                            g, b, s, a);
 }
 
 template <typename S>
@@ -442,17 +444,14 @@ cudaError_t launch_from_storage(const void *src, float *dst, long n, float wr, i
 
 cudaError_t launch_d3q19_stream_swap(const Pop<19> &p, const uint8_t *sb, int W, int H, int D,
                                      cudaStream_t s) {
-    d3q19_stream_swap_kernel<<<grid_of(W, H, D), D3_BLOCK, 0, s>>>(p, sb, W, H, D);
-    return cudaGetLastError();
+    return launch_dependent(d3q19_stream_swap_kernel, grid_of(W, H, D), dim3(D3_BLOCK), s, p, sb,
+                            W, H, D);
 }
 
 cudaError_t launch_d3q19_collide(const D3Args &a0, bool plot, cudaStream_t s) {
     const D3Args a = with_zou_he(a0);
-    if (plot)
-        d3q19_collide_kernel<true><<<grid_of(a.W, a.H, a.D), D3_BLOCK, 0, s>>>(a);
-    else
-        d3q19_collide_kernel<false><<<grid_of(a.W, a.H, a.D), D3_BLOCK, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(plot ? d3q19_collide_kernel<true> : d3q19_collide_kernel<false>,
+                            grid_of(a.W, a.H, a.D), dim3(D3_BLOCK), s, a);
 }
 
 cudaError_t launch_d3q19_get_border(const CPop<19> &p, const Pop<10> &b, int W, int H, int D,

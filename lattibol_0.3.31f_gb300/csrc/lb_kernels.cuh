@@ -105,18 +105,24 @@ __device__ __forceinline__ void after_predecessor() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s,
-                             const A &...args) {
+cudaError_t launch_dependent_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t s, const A &...args) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s,
+                             const A &...args) {
+    return launch_dependent_smem(kernel, grid, block, 0, s, args...);
 }
 
 // D3Q19

@@ -341,6 +341,7 @@ __global__ void __launch_bounds__((StageShape<S, TX>::THREADS), (StageShape<S, T
     auto issue = [&](int slot, int zs) {
         cp.issue(a, stage + slot * SS::ELEMS, &full[slot], zs);
     };
+    after_predecessor();  // barriers and chunk offsets are set up while it drains
     for (int j = 0; j < SS::SLOTS && j < nst; j++) issue(j, z0 - 1 + j);
 
     // step j: psi of plane z0 - 1 + j from its stage (the own nodes' populations
@@ -519,10 +520,9 @@ cudaError_t stage_launch(const D3Args &a, cudaStream_t s) {
     if (attr_e != cudaSuccess) return attr_e;
     const int nx = a.W / TX, ny = a.H / ST_TY;
     const int zc = chunk_planes((long)nx * ny, a.D, SS::MIN_BLOCKS);
-    d3q19_sc_stage_kernel<S, MOM, PSI, TX>
-        <<<dim3(nx, ny, (a.D + zc - 1) / zc), SS::THREADS, SS::SMEM, s>>>(
-            a, zc, ST_WAIT, pair_constants(), pair_d3<S>(a));
-    return cudaGetLastError();
+    return launch_dependent_smem(d3q19_sc_stage_kernel<S, MOM, PSI, TX>,
+                                 dim3(nx, ny, (a.D + zc - 1) / zc), dim3(SS::THREADS), SS::SMEM, s,
+                                 a, zc, ST_WAIT, pair_constants(), pair_d3<S>(a));
 }
 
 // 16-bit storage takes the wide tile where the width allows it (256^3: 53.9
