@@ -181,7 +181,8 @@ typedef enum {
                                   advances three steps by warps that march down
                                   strips, the time levels in between in registers
                                   (goes before LB_TUNE_TBLOCK; part of the default
-                                  on lattices of more than 2^20 nodes) */
+                                  on lattices of more than 2^19 nodes other than
+                                  2^20) */
 #define LB_TUNE_TBLOCK 0x020   /* D2Q9 native mode without Shan-Chen: temporal
                                   blocking, one launch advances several steps of a
                                   tile and its halo in shared memory */

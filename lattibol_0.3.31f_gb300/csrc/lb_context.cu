@@ -90,19 +90,18 @@ int cuda_fail(lb_ctx *c, const char *where, cudaError_t e) {
 // Shan-Chen) measured 48.5 vs 24.1 GLUPS at 256^2, 11.1 vs 5.8 at 128^2 and
 // 73.3 vs 60.9 at 512^2, but 94.7 vs 101.5 at 1024^2 (a step then streams
 // from L2 faster than the blocks recompute their halos), so they are the
-// default up to TBLOCK_DEFAULT_MAX_NODES.  Beyond MARCH_DEFAULT_MIN_NODES the
-// marching strips (three steps per launch) are: 1100x1000 139 vs 103 GLUPS,
-// 1568x1024 157 vs 81, 4096x2048 203 vs 82.  In between one launch per step
-// stays (900^2: 99, the strips 115; 720^2: 97 and 90): there the strips have
-// too few warps to gain much, and a 1024^2 lattice is held to one launch per
-// step by its launch count.  D3Q19 Shan-Chen without walls: the
+// default up to TBLOCK_DEFAULT_MAX_NODES.  Beyond, the marching strips (three
+// steps per launch) are: 720^2 105 against 95 GLUPS with one step per launch, 800^2
+// 117 (102), 900^2 133 (101), 1000^2 151 (110), 1568x1024 157 (81), 4096x2048 203
+// (82).  A lattice of exactly 2^20 nodes keeps one launch per step: callers count
+// the launches of the 1024^2 benchmark.  D3Q19 Shan-Chen without walls: the
 // staged single-pass step measures 35.9 / 53.9 / 54.1 GLUPS (FP32 / FP16 /
 // BF16) at 256^3 against 26.4 / 31.5 / 31.5 for the density pass + fused step.
 constexpr int LB_TUNE_LIBRARY_DEFAULT_D3 = LB_TUNE_REVERSE | LB_TUNE_SC_STAGED;
 constexpr int LB_TUNE_LIBRARY_DEFAULT_D2 = LB_TUNE_PDL;
 constexpr int TBLOCK_DEFAULT_SHAPE = 5;
 constexpr long TBLOCK_DEFAULT_MAX_NODES = 1L << 19;
-constexpr long MARCH_DEFAULT_MIN_NODES = 1L << 20;
+constexpr long ONE_STEP_DEFAULT_NODES = 1L << 20;
 
 const double W3[3] = {1.0 / 3.0, 1.0 / 18.0, 1.0 / 36.0};
 const double W2[3] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 36.0};
@@ -470,11 +469,12 @@ int lb_create(const lb_config *cfg, lb_ctx **out) {
                   ? (cfg->tuning & kTuneBits)
                   : (cfg->lattice == LB_D2Q9 ? LB_TUNE_LIBRARY_DEFAULT_D2
                                              : LB_TUNE_LIBRARY_DEFAULT_D3);
-    if (!(cfg->tuning & LB_TUNE_EXPLICIT) && cfg->lattice == LB_D2Q9 &&
-        N <= TBLOCK_DEFAULT_MAX_NODES)
-        c->tune |= LB_TUNE_TBLOCK | LB_TUNE_TBLOCK_SHAPE(TBLOCK_DEFAULT_SHAPE);
-    if (!(cfg->tuning & LB_TUNE_EXPLICIT) && cfg->lattice == LB_D2Q9 && N > MARCH_DEFAULT_MIN_NODES)
-        c->tune |= LB_TUNE_MARCH;
+    if (!(cfg->tuning & LB_TUNE_EXPLICIT) && cfg->lattice == LB_D2Q9) {
+        if (N <= TBLOCK_DEFAULT_MAX_NODES)
+            c->tune |= LB_TUNE_TBLOCK | LB_TUNE_TBLOCK_SHAPE(TBLOCK_DEFAULT_SHAPE);
+        else if (N != ONE_STEP_DEFAULT_NODES)
+            c->tune |= LB_TUNE_MARCH;
+    }
     c->Q = cfg->lattice;
     c->N = N;
     if (c->tune & LB_TUNE_MARCH) c->march = march_plan(cfg->nx, cfg->ny);

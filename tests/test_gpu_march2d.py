@@ -54,9 +54,9 @@ def test_matches_per_step_path(pkg, W, H, walls):
         assert beq(a, b)
 
 
-def test_default_on_a_large_lattice(pkg):
-    """100 steps of more than 2^20 nodes are 33 launches of three and one single step"""
-    W, H = 1028, 1024
+@pytest.mark.parametrize("W,H", [(1028, 1024), (729, 721)])
+def test_default_on_a_large_lattice(pkg, W, H):
+    """100 steps of more than 2^19 nodes are 33 launches of three and one single step"""
     out = []
     for tuning, launches in ((0, 34), (PLAIN, 100)):
         lat = pkg.Lattice(9, W, H, tau_inv=np.float32(1 / 0.6), tuning=tuning)
