@@ -160,9 +160,9 @@ __device__ __forceinline__ void d2q9_adhesion_sums(const uint8_t *s, int m1, int
     if (s[m8] & CELL_WALL) { Fsx = Fsx + w5; Fsy = Fsy + w5; }
 }
 
-template <int MODE, bool PLOT>
+template <int MODE, bool PLOT, bool DEP>
 __global__ void __launch_bounds__(D2_BLOCK) d2q9_sc_kernel(const D2Args a) {
-    after_predecessor();
+    if (DEP) after_predecessor();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= a.W) return;
@@ -308,6 +308,16 @@ __global__ void d2q9_equilibrium_kernel(Pop<9> p, const float *rho, const float 
 // ---------------------------------------------------------------- launchers
 static dim3 grid2(int W, int H) { return dim3((W + D2_BLOCK - 1) / D2_BLOCK, H); }
 
+// the Shan-Chen pass
+static cudaError_t launch_sc(const D2Args &a, int mode, bool plot, cudaStream_t s) {
+    const dim3 g = grid2(a.W, a.H), b(D2_BLOCK);
+#define LB_D2_SC(M, PL) \
+    launch_step(d2q9_sc_kernel<M, PL, true>, d2q9_sc_kernel<M, PL, false>, g, b, s, a)
+    if (mode == MODE_REF) return plot ? LB_D2_SC(MODE_REF, true) : LB_D2_SC(MODE_REF, false);
+    return plot ? LB_D2_SC(MODE_NATIVE, true) : LB_D2_SC(MODE_NATIVE, false);
+#undef LB_D2_SC
+}
+
 cudaError_t launch_d2q9_fused(const D2Args &a0, int mode, bool mom, bool plot, cudaStream_t s) {
     const D2Args a = with_zou_he(a0);
     const dim3 g = grid2(a.W, a.H), b(D2_BLOCK);
@@ -318,7 +328,8 @@ cudaError_t launch_d2q9_fused(const D2Args &a0, int mode, bool mom, bool plot, c
     if (sc) mom = true;  // the second pass reads rho
 #define LB_D2_CASE(M, MO, PL, SC)                                                 \
     if (mode == M && mom == MO && plot == PL && sc == SC) {                       \
-        e = PL || SC ? launch_dependent(d2q9_fused_kernel<M, MO, PL, SC, true>, g, b, s, a) \
+        e = PL || SC ? launch_step(d2q9_fused_kernel<M, MO, PL, SC, true>,      \
+                                   d2q9_fused_kernel<M, MO, PL, SC>, g, b, s, a) \
                      : (d2q9_fused_kernel<M, MO, PL, SC><<<g, b, 0, s>>>(a), cudaGetLastError()); \
         ok = true;                                                                \
     }
@@ -337,11 +348,7 @@ cudaError_t launch_d2q9_fused(const D2Args &a0, int mode, bool mom, bool plot, c
 #undef LB_D2_CASE
     if (!ok) return cudaErrorInvalidValue;
     if (e != cudaSuccess || !sc_pass) return e;
-    if (mode == MODE_REF)
-        return launch_dependent(plot ? d2q9_sc_kernel<MODE_REF, true>
-                                     : d2q9_sc_kernel<MODE_REF, false>, g, b, s, a);
-    return launch_dependent(plot ? d2q9_sc_kernel<MODE_NATIVE, true>
-                                 : d2q9_sc_kernel<MODE_NATIVE, false>, g, b, s, a);
+    return launch_sc(a, mode, plot, s);
 }
 
 cudaError_t launch_d2q9_fused_pdl(const D2Args &a0, int mode, bool mom, cudaStream_t s) {
@@ -368,8 +375,7 @@ cudaError_t launch_d2q9_collide(const D2Args &a0, bool plot, cudaStream_t s) {
     const cudaError_t e = launch_dependent(plot ? d2q9_collide_kernel<true>
                                                 : d2q9_collide_kernel<false>, g, b, s, a);
     if (e != cudaSuccess || !(a.G < 0.f)) return e;
-    return launch_dependent(plot ? d2q9_sc_kernel<MODE_REF, true>
-                                 : d2q9_sc_kernel<MODE_REF, false>, g, b, s, a);
+    return launch_sc(a, MODE_REF, plot, s);
 }
 
 cudaError_t launch_d2q9_get_border(const CPop<9> &p, const Pop<6> &b, int W, int H,

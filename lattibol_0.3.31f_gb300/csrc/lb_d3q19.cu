@@ -43,10 +43,11 @@ namespace lb {
 constexpr long FUSED_PF_BLOCKS = 912;
 static_assert(D3_BLOCK * 2 == 256, "two 128-byte lines per 16-bit population run");
 
-template <int MODE, bool MOM, bool PLOT, typename S, bool SC>
+// DEP: launched as a programmatic dependent (launch_step)
+template <int MODE, bool MOM, bool PLOT, typename S, bool SC, bool DEP>
 __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
     d3q19_fused_kernel(const D3Args a) {
-    after_predecessor();
+    if (DEP) after_predecessor();
     const Coord3 c(a);
     const int x = c.x, y = c.y, z = c.z;
     if (x >= a.W) return;
@@ -142,9 +143,9 @@ __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
 // Density pass of the Shan-Chen step: psi(rho) of the post-stream density of
 // every fluid node (the native moments' sum, so rho is the same float the
 // fused kernel computes), 0 at walls.
-template <typename S>
+template <typename S, bool DEP>
 __global__ void __launch_bounds__(D3_BLOCK) d3q19_density_kernel(const D3Args a) {
-    after_predecessor();
+    if (DEP) after_predecessor();
     const Coord3 c(a);
     if (c.x >= a.W) return;
     const int o = c.x + a.W * (c.y + a.H * c.z);
@@ -315,7 +316,8 @@ cudaError_t launch_d3q19_fused(const D3Args &a0, int mode, bool mom, bool plot, 
     const dim3 g = grid_of(a.W, a.H, a.D), b(D3_BLOCK);
 #define LB_D3_CASE(M, MO, PL)                                                    \
     if (mode == M && mom == MO && plot == PL) {                                  \
-        return launch_dependent(d3q19_fused_kernel<M, MO, PL, float, false>, g, b, s, a); \
+        return launch_step(d3q19_fused_kernel<M, MO, PL, float, false, true>, \
+                           d3q19_fused_kernel<M, MO, PL, float, false, false>, g, b, s, a); \
     }
     LB_D3_CASE(MODE_REF, true, true)
     LB_D3_CASE(MODE_REF, true, false)
@@ -329,16 +331,17 @@ cudaError_t launch_d3q19_fused(const D3Args &a0, int mode, bool mom, bool plot, 
 template <typename S>
 static cudaError_t native_launch(const D3Args &a, bool mom, bool sc, cudaStream_t s) {
     const dim3 g = grid_of(a.W, a.H, a.D), b(D3_BLOCK);
+#define LB_D3_STEP(MO, SC)                                                       \
+    launch_step(d3q19_fused_kernel<MODE_NATIVE, MO, false, S, SC, true>,         \
+                d3q19_fused_kernel<MODE_NATIVE, MO, false, S, SC, false>, g, b, s, a)
     if (sc) {
-        const cudaError_t e = launch_dependent(d3q19_density_kernel<S>, g, b, s, a);
+        const cudaError_t e =
+            launch_step(d3q19_density_kernel<S, true>, d3q19_density_kernel<S, false>, g, b, s, a);
         if (e != cudaSuccess) return e;
-        return launch_dependent(mom ? d3q19_fused_kernel<MODE_NATIVE, true, false, S, true>
-                                    : d3q19_fused_kernel<MODE_NATIVE, false, false, S, true>,
-                                g, b, s, a);
+        return mom ? LB_D3_STEP(true, true) : LB_D3_STEP(false, true);
     }
-    return launch_dependent(mom ? d3q19_fused_kernel<MODE_NATIVE, true, false, S, false>
-                                : d3q19_fused_kernel<MODE_NATIVE, false, false, S, false>,
-                            g, b, s, a);
+    return mom ? LB_D3_STEP(true, false) : LB_D3_STEP(false, false);
+#undef LB_D3_STEP
 }
 
 template <typename S>
@@ -349,8 +352,8 @@ static cudaError_t native_planes(const D3Args &a0, bool mom, int z_lo, int z_ski
     a.z_lo = z_lo;
     a.z_skip = z_skip;
     const dim3 g((a.W + D3_BLOCK - 1) / D3_BLOCK, a.H, nplanes), b(D3_BLOCK);
-    if (mom) d3q19_fused_kernel<MODE_NATIVE, true, false, S, false><<<g, b, 0, s>>>(a);
-    else d3q19_fused_kernel<MODE_NATIVE, false, false, S, false><<<g, b, 0, s>>>(a);
+    if (mom) d3q19_fused_kernel<MODE_NATIVE, true, false, S, false, false><<<g, b, 0, s>>>(a);
+    else d3q19_fused_kernel<MODE_NATIVE, false, false, S, false, false><<<g, b, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -125,6 +125,23 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
     return launch_dependent_smem(kernel, grid, block, 0, s, args...);
 }
 
+// One of a step's kernels, one thread per node: a dependent launch where the
+// start of a launch weighs, on grids of up to 2432 blocks (16 per SM, one wave),
+// and on the legacy default stream, which runs beside no other.  Three lattices
+// side by side, GLUPS without and with: 45 x 23 x 17 7.4, 10.5; 100 x 45 x 40 49, 61;
+// 16 x 13 x 187 (2431 blocks) 14.2, 15.6; beyond, 64^3 46, 53, but 30 x 64 x 64 36, 29
+// and 120 x 40 x 100 46.9, 46.3: on grids of short blocks after_predecessor itself
+// costs (30 x 157 x 126 in FP16, 19 782 blocks: 26, 16), so `plain` is the kernel
+// without it.
+template <typename Args>
+cudaError_t launch_step(void (*dependent)(Args), void (*plain)(Args), dim3 grid, dim3 block,
+                        cudaStream_t s, const Args &a) {
+    if (s == nullptr || (long)grid.x * grid.y * grid.z <= 2432)
+        return launch_dependent(dependent, grid, block, s, a);
+    plain<<<grid, block, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
 // D3Q19
 cudaError_t launch_d3q19_fused(const D3Args &a, int mode, bool mom, bool plot, cudaStream_t s);
 // native mode with storage kind (0 f32, 1 f16, 2 bf16) and optional Shan-Chen
