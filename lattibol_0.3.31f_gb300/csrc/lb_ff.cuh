@@ -12,6 +12,8 @@
 // bound was made for, the FP64 line itself runs.  Same bits, on every input.
 #pragma once
 
+#include <cmath>
+
 #include <cuda_runtime.h>
 
 namespace lb {
@@ -35,12 +37,32 @@ __device__ __forceinline__ bool ff_round(float s, float lo, float bound, float &
     return out == s + (lo - bound) && fabsf(out) > 1e-28f;
 }
 
+// 1 / x within 1 ulp, from the hardware (a host model of these forms brings its own)
+#ifdef __CUDACC__
+__device__ __forceinline__ float ff_rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+#else
+float ff_rcp(float x);
+#endif
+
 // a positive constant as two floats (48 bits)
 struct FF {
     float hi, lo;
 };
 __host__ __device__ constexpr FF ff_const(double v) {
     return FF{(float)v, (float)(v - (double)(float)v)};
+}
+// 1 / v as two floats, for ff_ratio.  The low part of a quotient below 2^-100 may
+// lie among the subnormal floats and keep fewer bits than ff_ratio's bound allows
+// for (v = 1e34: 1 result in 26 rounded the wrong way); such a pair is not a
+// number, on which ff_ratio leaves the value to the FP64 line.
+inline FF ff_reciprocal(double v) {
+    const double r = 1. / v;
+    if (r < 0x1p-100 && r > -0x1p-100) return FF{NAN, NAN};
+    return ff_const(r);
 }
 
 // 4 exp(-200 / rho) rounded to float, for rho in [8, 2^20].  The quotient by its
@@ -50,8 +72,7 @@ __host__ __device__ constexpr FF ff_const(double v) {
 // 2^-37; the bound is 2^-35, so about one value in 2^10 takes the FP64 line.
 __device__ __forceinline__ bool ff_psi_ref(float rho, float &out) {
     if (!(rho >= 8.f && rho <= 1048576.f)) return false;
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(rho));
+    float y = ff_rcp(rho);
     y = __fmaf_rn(y, __fmaf_rn(-rho, y, 1.f), y);
     const float q = -200.f * y;
     const float q_lo = __fmaf_rn(-q, rho, -200.f) * y;  // exact remainder over rho
@@ -108,7 +129,7 @@ __device__ __forceinline__ bool ff_face(float base, FF c, float ru, float t2, fl
 }
 
 // (float)(add + ((double)a + 2 (double)b) inv), inv = 1 / (1 - ux) or 1 / rho_out
-// to 48 bits: the density and velocity of a Zou-He face
+// to 48 bits (ff_reciprocal): the density and velocity of a Zou-He face
 __device__ __forceinline__ bool ff_ratio(float a, float b, FF inv, float add, float &out) {
     float e0, e1, e2;
     const float n = ff_sum(a, 2.f * b, e0);

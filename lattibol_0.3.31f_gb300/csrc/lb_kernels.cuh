@@ -90,8 +90,8 @@ struct D2Args {
 // the arguments with the reference mode's Zou-He reciprocals
 template <typename Args> Args with_zou_he(const Args &a0) {
     Args a = a0;
-    a.inv_in = ff_const(1. / (1. - (double)a.ux_in));
-    a.inv_out = ff_const(1. / (double)a.rho_out);
+    a.inv_in = ff_reciprocal(1. - (double)a.ux_in);
+    a.inv_out = ff_reciprocal((double)a.rho_out);
     return a;
 }
 
