@@ -32,4 +32,25 @@ long ratio_wrong(const float *a, const float *b, long n, double v, float add) {
     return wrong;
 }
 
+// every `step`-th float of [lo, hi], the reciprocal's seed off by -1, 0 and +1 ulp:
+// the largest relative error of the two floats of 4 exp(-200 / rho), and how many
+// of the values that the form decides differ from the FP64 line
+double psi_error(float lo, float hi, int step, long *wrong) {
+    double worst = 0;
+    *wrong = 0;
+    for (seed_ulps = -1; seed_ulps <= 1; seed_ulps++)
+        for (int i = __float_as_int(lo); i <= __float_as_int(hi); i += step) {
+            const float rho = __int_as_float(i);
+            float h, l, out;
+            if (!lb::ff_psi_parts(rho, h, l)) return INFINITY;
+            // the FP64 line's own error, 2^-52 or so, does not show at 2^-35
+            const double line = 4. * exp(-200. / (double)rho);
+            worst = fmax(worst, fabs(((double)h + (double)l - line) / line));
+            const float f = (float)line;
+            if (lb::ff_psi_ref(rho, out)) *wrong += memcmp(&f, &out, 4) != 0;
+        }
+    seed_ulps = 0;
+    return worst;
+}
+
 }

@@ -18,6 +18,7 @@ def host(tmp_path_factory):
                     "-I" + cuda, os.path.join(HERE, "ff_host.cpp"), "-o", out], check=True)
     lib = ctypes.CDLL(out)
     lib.ratio_wrong.restype = ctypes.c_long
+    lib.psi_error.restype = ctypes.c_double
     return lib
 
 
@@ -36,3 +37,18 @@ def test_face_quotients(host, v, add):
     a, b = (np.float32(v) * rng.uniform(0.1, 0.9, (2, n))).astype(np.float32)
     assert host.ratio_wrong(ptr(a), ptr(b), ctypes.c_long(n), ctypes.c_double(v),
                             ctypes.c_float(add)) == 0
+
+
+# a sweep over the whole range, and every float where the reduced argument is at
+# its largest for several k (rho = 200 / ((k + 1/2) ln 2))
+@pytest.mark.parametrize("lo,hi,step", [(8.0, 2.0 ** 20, 61)] + [
+    (200 / ((k + 0.5) * np.log(2)) * (1 - 2e-3), 200 / ((k + 0.5) * np.log(2)) * (1 + 2e-3), 1)
+    for k in (0, 1, 2, 5, 12, 20, 35)])
+def test_psi(host, lo, hi, step):
+    """the form's error is at most half of what its rounding check allows (2^-35), and
+    no value that the check decides differs from the FP64 line"""
+    wrong = ctypes.c_long()
+    err = host.psi_error(ctypes.c_float(lo), ctypes.c_float(hi), ctypes.c_int(step),
+                         ctypes.byref(wrong))
+    assert wrong.value == 0
+    assert err <= 2.0 ** -36, np.log2(err)
