@@ -42,7 +42,8 @@ struct lb_ctx {
     float wr[19] = {0};                  // 16-bit storage offsets w_k * rho_ref
     int tune = 0;                        // LB_TUNE_* bits in effect
     MarchPlan march{};                   // marching strips: the items of a launch
-    uint16_t *wmask = nullptr;           // and their upstream-wall masks
+    uint16_t *wmask = nullptr;           // and their upstream-wall masks,
+    bool wmask_ok = false;               // those of the present flags
     bool closure_on = false;             // learned closure sets the local relaxation time
     ClosureArgs closure{};
     bool flags_set = false;
@@ -170,10 +171,12 @@ int tblock_variant(const lb_ctx *c) {
 }
 
 // the marching strips advance a launch of march_steps_per_launch() steps: D2Q9
-// native mode without Shan-Chen, and the tuning asks for them
-bool march_on(const lb_ctx *c) {
+// native mode without Shan-Chen, and the tuning asks for them; lattices with walls
+// need the masks
+bool march_wanted(const lb_ctx *c) {
     return c->Q == 9 && !sc_on(c) && c->cfg.mode == LB_MODE_NATIVE && (c->tune & LB_TUNE_MARCH);
 }
+bool march_on(const lb_ctx *c) { return march_wanted(c) && (!c->any_wall || c->wmask_ok); }
 
 // steps per launch of the multi-step kernel in effect (0: one launch per step)
 int multi_steps(const lb_ctx *c) {
@@ -187,11 +190,22 @@ int multi_graph_launches(const lb_ctx *c, int steps_per_launch) {
     return std::max(2, (c->cfg.graph_steps / steps_per_launch) & ~1);
 }
 
-// the marching strips' upstream-wall masks after the flags changed
+// the marching strips' upstream-wall masks after the flags changed; where there is
+// no memory for them a lattice with walls takes one step per launch
 int update_wall_mask(lb_ctx *c, const char *where) {
-    if (!c->any_wall || !march_on(c)) return LB_OK;
-    if (!c->wmask) LB_TRY(c, where, cudaMalloc(&c->wmask, sizeof(uint16_t) * c->stride));
+    c->wmask_ok = false;
+    if (!c->any_wall || !march_wanted(c)) return LB_OK;
+    if (!c->wmask) {
+        const cudaError_t e = cudaMalloc(&c->wmask, sizeof(uint16_t) * c->stride);
+        if (e != cudaSuccess) c->wmask = nullptr;
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return LB_OK;
+        }
+        LB_TRY(c, where, e);
+    }
     LB_TRY(c, where, launch_d2q9_wall_mask(c->flags, c->wmask, c->cfg.nx, c->cfg.ny, c->stream));
+    c->wmask_ok = true;
     return LB_OK;
 }
 
@@ -558,11 +572,12 @@ int lb_set_flags(lb_ctx *c, const uint8_t *flags) {
     c->flags_set = true;
     bool any_wall = false;
     for (long o = 0; o < c->N && !any_wall; o++) any_wall = (f[o] & CELL_WALL) != 0;
-    if (any_wall != c->any_wall) drop_graphs(c);  // the step kernel may change
+    const int steps = multi_steps(c);
+    const bool had_wall = c->any_wall;
     c->any_wall = any_wall;
     const int rc = update_wall_mask(c, "lb_set_flags");
-    if (rc != LB_OK) return rc;
-    return LB_OK;
+    if (any_wall != had_wall || multi_steps(c) != steps) drop_graphs(c);  // another step kernel
+    return rc;
 }
 
 // populations cross the API as float; 16-bit storage converts on the device
