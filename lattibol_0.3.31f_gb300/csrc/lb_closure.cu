@@ -1056,24 +1056,13 @@ int mlp_gradient(lb_mlp *m, const float *X, const float *Z, long n, float *loss_
     const long chunks = (n + 127) / 128;
     const int nb = (int)std::min<long>(m->nblocks, chunks);
     // both as programmatic dependents of the launch before them
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nb);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = net::TRAIN_SMEM;
-    cfg.stream = m->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    LB_MTRY(m, "mlp_tc_kernel", cudaLaunchKernelEx(&cfg, mlp_tc_kernel<true>, mlp_dev(m), X, Z, n,
-                                                   m->partial, m->err_dev));
-    cfg.gridDim = dim3((NGRAD + RED_PAR - 1) / RED_PAR);
-    cfg.blockDim = dim3(RED_PAR * RED_RUNS);
-    cfg.dynamicSmemBytes = 0;
-    LB_MTRY(m, "grad_reduce_kernel", cudaLaunchKernelEx(&cfg, grad_reduce_kernel,
-                                                        (const float *)m->partial, nb, m->grad,
-                                                        loss_slot, ad));
+    LB_MTRY(m, "mlp_tc_kernel",
+            launch_dependent_smem(mlp_tc_kernel<true>, dim3(nb), dim3(256), net::TRAIN_SMEM,
+                                  m->stream, mlp_dev(m), X, Z, n, m->partial, m->err_dev));
+    LB_MTRY(m, "grad_reduce_kernel",
+            launch_dependent(grad_reduce_kernel, dim3((NGRAD + RED_PAR - 1) / RED_PAR),
+                             dim3(RED_PAR * RED_RUNS), m->stream, m->partial, nb, m->grad,
+                             loss_slot, ad));
     return LB_OK;
 }
 

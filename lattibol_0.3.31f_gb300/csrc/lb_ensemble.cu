@@ -626,22 +626,11 @@ cudaError_t ens_pair_launch(lb_ensemble *e, int from, int steps, bool mom) {
     pa.a = args_for(e, from);
     pa.rows = e->pair_rows;
     pa.c = pair_constants();
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(e->nitems);
-    cfg.blockDim = dim3(32);
-    cfg.dynamicSmemBytes = EP_RING * EP_ROW * sizeof(float2);
-    cfg.stream = e->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     e->launches += 1;
-    if (steps == 1)
-        return mom ? cudaLaunchKernelEx(&cfg, ens_pair_kernel<1, true>, pa)
-                   : cudaLaunchKernelEx(&cfg, ens_pair_kernel<1, false>, pa);
-    return mom ? cudaLaunchKernelEx(&cfg, ens_pair_kernel<2, true>, pa)
-               : cudaLaunchKernelEx(&cfg, ens_pair_kernel<2, false>, pa);
+    const auto kernel = steps == 1 ? (mom ? ens_pair_kernel<1, true> : ens_pair_kernel<1, false>)
+                                   : (mom ? ens_pair_kernel<2, true> : ens_pair_kernel<2, false>);
+    return launch_dependent_smem(kernel, dim3(e->nitems), dim3(32),
+                                 EP_RING * EP_ROW * sizeof(float2), e->stream, pa);
 }
 
 // one step (any form)

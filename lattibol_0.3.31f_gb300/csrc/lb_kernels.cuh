@@ -117,7 +117,11 @@ cudaError_t launch_dependent_smem(void (*kernel)(P...), dim3 grid, dim3 block, s
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    // cudaLaunchKernelEx leaves its error behind as well as returning it: taken back
+    // here, so that the next launch's check does not report a refused one
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s,

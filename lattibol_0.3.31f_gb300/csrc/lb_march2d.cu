@@ -286,20 +286,12 @@ namespace {
 
 template <bool MOM, bool WALLS>
 cudaError_t md_launch(const MarchArgs &ma, cudaStream_t s) {
-    const D2Args &a = ma.a;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ma.items);
-    cfg.blockDim = dim3(32);
-    cfg.dynamicSmemBytes = MD_IN * MD_ROW * sizeof(float2);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (a.W % 4 == 0) return cudaLaunchKernelEx(&cfg, d2q9_march_kernel<MOM, WALLS, 4>, ma);
-    return a.W % 2 == 0 ? cudaLaunchKernelEx(&cfg, d2q9_march_kernel<MOM, WALLS, 2>, ma)
-                        : cudaLaunchKernelEx(&cfg, d2q9_march_kernel<MOM, WALLS, 1>, ma);
+    const int W = ma.a.W;
+    const auto kernel = W % 4 == 0   ? d2q9_march_kernel<MOM, WALLS, 4>
+                        : W % 2 == 0 ? d2q9_march_kernel<MOM, WALLS, 2>
+                                     : d2q9_march_kernel<MOM, WALLS, 1>;
+    return launch_dependent_smem(kernel, dim3(ma.items), dim3(32),
+                                 MD_IN * MD_ROW * sizeof(float2), s, ma);
 }
 
 }  // namespace

@@ -180,17 +180,8 @@ cudaError_t tb_launch(const D2Args &a, bool mom, cudaStream_t s) {
         cudaFuncSetAttribute(d2q9_tblock_kernel<TS, BX, BY, NT, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)};
     if (attr_e[mom ? 1 : 0] != cudaSuccess) return attr_e[mom ? 1 : 0];
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((a.W + BX - 1) / BX, (a.H + BY - 1) / BY);
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, a);
+    return launch_dependent_smem(kern, dim3((a.W + BX - 1) / BX, (a.H + BY - 1) / BY), dim3(NT),
+                                 smem, s, a);
 }
 
 }  // namespace
