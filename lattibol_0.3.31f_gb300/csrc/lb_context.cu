@@ -172,9 +172,13 @@ int tblock_variant(const lb_ctx *c) {
 
 // the marching strips advance a launch of march_steps_per_launch() steps: D2Q9
 // native mode without Shan-Chen, and the tuning asks for them; lattices with walls
-// need the masks
+// need the masks.  The masks' kernel and the single steps of a remainder take one
+// grid row per lattice row: a lattice of more rows than that is left to the
+// single-step launch, which refuses it whole.
+constexpr int MARCH_MAX_ROWS = 65535;
 bool march_wanted(const lb_ctx *c) {
-    return c->Q == 9 && !sc_on(c) && c->cfg.mode == LB_MODE_NATIVE && (c->tune & LB_TUNE_MARCH);
+    return c->Q == 9 && !sc_on(c) && c->cfg.mode == LB_MODE_NATIVE && (c->tune & LB_TUNE_MARCH) &&
+           c->cfg.ny <= MARCH_MAX_ROWS;
 }
 bool march_on(const lb_ctx *c) { return march_wanted(c) && (!c->any_wall || c->wmask_ok); }
 
