@@ -181,8 +181,9 @@ typedef enum {
                                   advances three steps by warps that march down
                                   strips, the time levels in between in registers
                                   (goes before LB_TUNE_TBLOCK; part of the default
-                                  on lattices of more than 2^19 nodes other than
-                                  2^20) */
+                                  on lattices of more than 2^19 nodes, except those
+                                  of exactly 2^20 and those of so few rows, under
+                                  32, that one step per launch is faster) */
 #define LB_TUNE_TBLOCK 0x020   /* D2Q9 native mode without Shan-Chen: temporal
                                   blocking, one launch advances several steps of a
                                   tile and its halo in shared memory */

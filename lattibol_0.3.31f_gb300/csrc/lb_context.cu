@@ -92,10 +92,14 @@ int cuda_fail(lb_ctx *c, const char *where, cudaError_t e) {
 // 73.3 vs 60.9 at 512^2, but 94.7 vs 101.5 at 1024^2 (a step then streams
 // from L2 faster than the blocks recompute their halos), so they are the
 // default up to TBLOCK_DEFAULT_MAX_NODES.  Beyond, the marching strips (three
-// steps per launch) are: 720^2 105 against 95 GLUPS with one step per launch, 800^2
-// 117 (102), 900^2 133 (101), 1000^2 151 (110), 1568x1024 157 (81), 4096x2048 203
-// (82).  A lattice of exactly 2^20 nodes keeps one launch per step: callers count
-// the launches of the 1024^2 benchmark.  D3Q19 Shan-Chen without walls: the
+// steps per launch) are, where march_pays.  Around the line (GLUPS of the strips, of
+// the blocks in brackets, no walls; the same with 5 % walls): 600^2 82 (94), 62 (65);
+// 640^2 87 (92), 64 (64); 700^2 106 (96), 78 (67); 728x724 103 (104), 76 (72); 800^2
+// 117 (103), 85 (71).  One launch per step: 102 at 800^2, 106 at 1000^2 (strips 150),
+// 81 at 1568x1024 (175), 82 at 4096x2048 (203).  A lattice of exactly 2^20 nodes keeps
+// one launch per step although the strips are faster there too (1024^2: 107, strips
+// 149): tests/test_gpu_tblock.py holds the default to one launch per step at 1024^2.
+// D3Q19 Shan-Chen without walls: the
 // staged single-pass step measures 35.9 / 53.9 / 54.1 GLUPS (FP32 / FP16 /
 // BF16) at 256^3 against 26.4 / 31.5 / 31.5 for the density pass + fused step.
 constexpr int LB_TUNE_LIBRARY_DEFAULT_D3 = LB_TUNE_REVERSE | LB_TUNE_SC_STAGED;
@@ -490,7 +494,7 @@ int lb_create(const lb_config *cfg, lb_ctx **out) {
     if (!(cfg->tuning & LB_TUNE_EXPLICIT) && cfg->lattice == LB_D2Q9) {
         if (N <= TBLOCK_DEFAULT_MAX_NODES)
             c->tune |= LB_TUNE_TBLOCK | LB_TUNE_TBLOCK_SHAPE(TBLOCK_DEFAULT_SHAPE);
-        else if (N != ONE_STEP_DEFAULT_NODES)
+        else if (N != ONE_STEP_DEFAULT_NODES && march_pays(cfg->nx, cfg->ny))
             c->tune |= LB_TUNE_MARCH;
     }
     c->Q = cfg->lattice;

@@ -206,8 +206,10 @@ cudaError_t launch_d2q9_tblock(const D2Args &a, int variant, bool mom, cudaStrea
 // launch_d2q9_wall_mask's (N values, on 4 bytes), null on a lattice without walls
 struct MarchPlan {
     int tw, rows, strips, items;  // columns and rows of an item; strips; items
+    double us;                    // estimated time per step
 };
 MarchPlan march_plan(int W, int H);
+bool march_pays(int W, int H);  // faster than one launch per step
 int march_steps_per_launch();
 cudaError_t launch_d2q9_march(const D2Args &a, const MarchPlan &p, const uint16_t *mask, bool mom,
                               cudaStream_t s);

@@ -302,8 +302,8 @@ int march_steps_per_launch() { return T; }
 // rows that an item reads beyond its own.  A pass takes an item's march times a
 // function of the rounds of items w (a partly filled round runs its warps
 // faster, a nearly empty second one costs almost as much as a full one;
-// measured at 1568 x 1024: 16 rows, 1792 items for 1824 warps, 1.20 ms per 100
-// steps; 12 rows 1.48, 24 rows 1.41, 32 rows 1.68).
+// measured at 1568 x 1024, us per step: 16 rows, 1792 items for 1824 warps, 12.0;
+// 12 rows 14.8, 24 rows 14.1, 32 rows 16.8).
 MarchPlan march_plan(int W, int H) {
     MarchPlan p{};
     const int ns = (W + MD_COLS - 1) / MD_COLS;
@@ -322,7 +322,27 @@ MarchPlan march_plan(int W, int H) {
         }
     }
     p.items = p.strips * ((H + p.rows - 1) / p.rows);
+    // us per step: the upper end of what lattices of 0.53 .. 2.7 M nodes without walls
+    // and of 3 .. 100 rows gave.  Up to one round of items it is one march, whatever w
+    // (odd widths 0.43 .. 0.48 per row, others 0.36 .. 0.42); beyond, it follows the cost
+    // (0.43 .. 0.50, 0.38 .. 0.46).
+    const bool odd = W % 2 != 0;
+    p.us = p.items <= warps ? (p.rows + 2 * T) * (odd ? 0.48 : 0.41) : best * (odd ? 0.50 : 0.45);
     return p;
+}
+
+// Whether the strips beat one launch per step (beyond 2^19 nodes).  From 32 rows on
+// they did on every shape measured (1.02 to 2.5 times; 135 shapes of 0.53 .. 2.7 M
+// nodes, with rows that start on 4, 8 and 16 bytes).  On fewer rows the 2 T rows that
+// an item reads beyond its own can outweigh it: us per step, strips / one launch per
+// step, 700 001 x 1 17.6 / 6.4, 175 000 x 4 7.8 / 6.6, 53 125 x 16 9.9 / 8.2, but
+// 50 001 x 20 7.5 / 9.7 and 525 000 x 4 19.5 / 25.4.  There the plan's time is compared
+// with that of a launch per step, 0.3 us and 9.5 ps per thread (blocks of 128 along a
+// row), 11.5 beyond 1.6 M threads, where the two population sets leave L2.
+bool march_pays(int W, int H) {
+    if (H >= 32) return true;
+    const double threads = 128. * ((W + 127) / 128) * H;
+    return march_plan(W, H).us < 0.3 + threads * (threads > 1.6e6 ? 11.5e-6 : 9.5e-6);
 }
 
 cudaError_t launch_d2q9_march(const D2Args &a, const MarchPlan &p, const uint16_t *mask, bool mom,

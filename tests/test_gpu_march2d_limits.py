@@ -25,3 +25,26 @@ def test_more_rows_than_a_grid_takes(pkg, walls, tuning):
         assert lat.steps_done() == 0
     assert np.array_equal(f.view(np.uint32), lat.populations().view(np.uint32))
     lat.close()
+
+
+@pytest.mark.parametrize("W,H,launches", [(700001, 1, 6), (263000, 2, 6), (140000, 5, 6),
+                                          (53125, 16, 6), (50001, 20, 2), (525000, 4, 2),
+                                          (17000, 32, 2), (729, 721, 2)])
+def test_lattices_of_few_rows(pkg, W, H, launches):
+    """six steps by default: two launches of three where the strips are the faster form,
+    six where the rows an item reads beyond its own outweigh them; the same bits"""
+    N = W * H
+    rng = np.random.default_rng(2)
+    rho = (1 + 0.01 * rng.standard_normal(N)).astype(np.float32)
+    out = []
+    for tuning in (0, 0x108):
+        lat = pkg.Lattice(9, W, H, tau_inv=np.float32(1 / 0.6), tuning=tuning)
+        lat.set_flags(np.zeros(N, np.uint8))
+        lat.init_equilibrium(rho)
+        before = lat.launches()
+        lat.step(6)
+        if tuning == 0:
+            assert lat.launches() - before == launches
+        out.append(lat.populations())
+        lat.close()
+    assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
