@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
 // Density pass of the Shan-Chen step: psi(rho) of the post-stream density of
 // every fluid node (the native moments' sum, so rho is the same float the
 // fused kernel computes), 0 at walls.
-template <typename S, bool DEP>
+template <typename S, int PSI, bool DEP>
 __global__ void __launch_bounds__(D3_BLOCK) d3q19_density_kernel(const D3Args a) {
     if (DEP) after_predecessor();
     const Coord3 c(a);
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(D3_BLOCK) d3q19_density_kernel(const D3Args a)
     float g[19];
     pull_native<S>(a, o, n, fl, g);
     const float rho = StepArith<S>::rho(g, a);
-    a.psi[o] = a.psi_form == 0 ? psi_ref(rho) : psi_exp1(rho);
+    a.psi[o] = psi_form<PSI>(rho);
 }
 
 
@@ -336,7 +336,9 @@ static cudaError_t native_launch(const D3Args &a, bool mom, bool sc, cudaStream_
                 d3q19_fused_kernel<MODE_NATIVE, MO, false, S, SC, false>, g, b, s, a)
     if (sc) {
         const cudaError_t e =
-            launch_step(d3q19_density_kernel<S, true>, d3q19_density_kernel<S, false>, g, b, s, a);
+            a.psi_form == 0
+                ? launch_step(d3q19_density_kernel<S, 0, true>, d3q19_density_kernel<S, 0, false>, g, b, s, a)
+                : launch_step(d3q19_density_kernel<S, 1, true>, d3q19_density_kernel<S, 1, false>, g, b, s, a);
         if (e != cudaSuccess) return e;
         return mom ? LB_D3_STEP(true, true) : LB_D3_STEP(false, true);
     }

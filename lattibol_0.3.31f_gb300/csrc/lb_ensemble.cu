@@ -71,6 +71,7 @@ __device__ __forceinline__ void ens_pull(const EnsArgs &a, const EnsItem &dm, in
 
 // Both passes walk the work list with a stride of the grid size and load the
 // next item while they work on the current one.
+template <int PSI>
 __global__ void ens_density_kernel(const EnsArgs a) {
     int it = blockIdx.x;
     if (it >= a.nitems) return;
@@ -84,7 +85,7 @@ __global__ void ens_density_kernel(const EnsArgs a) {
                 float g[9];
                 ens_pull(a, dm, x, y, g);
                 const float rho = d2q9_rho_native(g);
-                a.psi[dm.off + x + dm.W * y] = a.psi_form == 0 ? psi_ref(rho) : psi_exp1(rho);
+                a.psi[dm.off + x + dm.W * y] = psi_form<PSI>(rho);
             }
         }
         dm = next;
@@ -150,7 +151,7 @@ __device__ __forceinline__ int ens_wrap(int v, int n, bool small) {
 
 // tiles of ET_BX x BY nodes, one thread per tile node; MINB resident blocks
 // per SM bound the registers
-template <int BY, int MINB, bool MOM>
+template <int BY, int MINB, bool MOM, int PSI>
 __global__ void __launch_bounds__(ET_BX * BY, MINB) ens_tile_kernel(const EnsArgs a) {
     constexpr int PY = BY + 2, RING = 2 * ET_PX + 2 * BY;
     // two psi tiles used by alternate items: a block passes one barrier per
@@ -187,10 +188,9 @@ __global__ void __launch_bounds__(ET_BX * BY, MINB) ens_tile_kernel(const EnsArg
                      ens_wrap(dm.y - 1 + ry, dm.H, small), g2);
         float rho, ux, uy;
         d2q9_moments_native(g, rho, ux, uy);
-        sp[ty + 1][tx + 1] = a.psi_form == 0 ? psi_ref(rho) : psi_exp1(rho);
+        sp[ty + 1][tx + 1] = psi_form<PSI>(rho);
         if (ring) {
-            const float r2 = d2q9_rho_native(g2);
-            sp[ry][rx] = a.psi_form == 0 ? psi_ref(r2) : psi_exp1(r2);
+            sp[ry][rx] = psi_form<PSI>(d2q9_rho_native(g2));
         }
         __syncthreads();
         if (dm.x + tx < dm.W && dm.y + ty < dm.H) {
@@ -222,12 +222,8 @@ __global__ void __launch_bounds__(ET_BX * BY, MINB) ens_tile_kernel(const EnsArg
 // ---------------------------------------------------------------------------
 constexpr int ENS_MARCH_THREADS = 256;
 
-__device__ __forceinline__ float ens_psi(const EnsArgs &a, float rho) {
-    return a.psi_form == 0 ? psi_ref(rho) : psi_exp1(rho);
-}
-
 // one strip item (march of R rows of 32 columns) by one warp, plain loads
-template <int R, bool MOM>
+template <int R, bool MOM, int PSI>
 __device__ __forceinline__ void ens_march_item(const EnsArgs &a, const EnsItem dm, int lane) {
     constexpr unsigned FULL = 0xffffffffu;
     const bool edge = lane == 0 || lane == 31;
@@ -242,15 +238,15 @@ __device__ __forceinline__ void ens_march_item(const EnsArgs &a, const EnsItem d
         float g[9];
         const int ym = ens_wrap(dm.y - 1, dm.H, false);
         ens_pull(a, dm, x, ym, g);
-        pm = ens_psi(a, d2q9_rho_native(g));
+        pm = psi_form<PSI>(d2q9_rho_native(g));
         ens_pull(a, dm, x, dm.y, gc);
         d2q9_moments_native(gc, rc, uxc, uyc);
-        pc = ens_psi(a, rc);
+        pc = psi_form<PSI>(rc);
         if (edge) {
             ens_pull(a, dm, xh, ym, g);
-            hm = ens_psi(a, d2q9_rho_native(g));
+            hm = psi_form<PSI>(d2q9_rho_native(g));
             ens_pull(a, dm, xh, dm.y, g);
-            hc = ens_psi(a, d2q9_rho_native(g));
+            hc = psi_form<PSI>(d2q9_rho_native(g));
         }
     }
     for (int r = dm.y; r < y_end; r++) {
@@ -260,10 +256,10 @@ __device__ __forceinline__ void ens_march_item(const EnsArgs &a, const EnsItem d
         if (edge) {
             float g[9];
             ens_pull(a, dm, xh, yp, g);
-            hn = ens_psi(a, d2q9_rho_native(g));
+            hn = psi_form<PSI>(d2q9_rho_native(g));
         }
         d2q9_moments_native(gn, rn, uxn, uyn);
-        const float pn = ens_psi(a, rn);
+        const float pn = psi_form<PSI>(rn);
         // x - 1 and x + 1 from the neighbour lanes, the halo at the strip ends
         float lm = __shfl_up_sync(FULL, pm, 1), lc = __shfl_up_sync(FULL, pc, 1);
         float ln = __shfl_up_sync(FULL, pn, 1);
@@ -290,14 +286,14 @@ __device__ __forceinline__ void ens_march_item(const EnsArgs &a, const EnsItem d
     }
 }
 
-template <int R, int MINB, bool MOM>
+template <int R, int MINB, bool MOM, int PSI>
 __global__ void __launch_bounds__(ENS_MARCH_THREADS, MINB) ens_march_kernel(const EnsArgs a) {
     const int lane = threadIdx.x & 31;
     const int warps_per_block = ENS_MARCH_THREADS / 32;
     const int nwarps = gridDim.x * warps_per_block;
     for (int it = blockIdx.x * warps_per_block + (threadIdx.x >> 5); it < a.nitems;
          it += nwarps)
-        ens_march_item<R, MOM>(a, a.items[it], lane);
+        ens_march_item<R, MOM, PSI>(a, a.items[it], lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -637,20 +633,27 @@ cudaError_t ens_pair_launch(lb_ensemble *e, int from, int steps, bool mom) {
 cudaError_t ens_step(lb_ensemble *e, int from, bool mom) {
     if (ens_pairs(e->shape)) return ens_pair_launch(e, from, 1, mom);
     const EnsArgs a = args_for(e, from);
+    const bool ref = e->psi_form == LB_PSI_REF;
     const unsigned grid = (unsigned)std::max(1, std::min(e->nitems, e->sms * e->shape.bps));
     if (e->shape.bx == 0) {
         switch (e->shape.ry) {
-#define LB_ENS_LAUNCH(S, BY, MINB)                                                            \
-    case S:                                                                                   \
-        if (mom) ens_tile_kernel<BY, MINB, true><<<grid, ET_BX * BY, 0, e->stream>>>(a);    \
-        else ens_tile_kernel<BY, MINB, false><<<grid, ET_BX * BY, 0, e->stream>>>(a);       \
+#define LB_ENS_LAUNCH(S, BY, MINB)                                                             \
+    case S:                                                                                    \
+        (ref ? mom ? ens_tile_kernel<BY, MINB, true, LB_PSI_REF>                               \
+                   : ens_tile_kernel<BY, MINB, false, LB_PSI_REF>                              \
+             : mom ? ens_tile_kernel<BY, MINB, true, LB_PSI_EXP1>                              \
+                   : ens_tile_kernel<BY, MINB, false, LB_PSI_EXP1>)                            \
+            <<<grid, ET_BX * BY, 0, e->stream>>>(a);                                           \
         break;
             LB_ENS_TILES(LB_ENS_LAUNCH)
 #undef LB_ENS_LAUNCH
 #define LB_ENS_MLAUNCH(S, R, MINB)                                                             \
     case S:                                                                                    \
-        if (mom) ens_march_kernel<R, MINB, true><<<grid, ENS_MARCH_THREADS, 0, e->stream>>>(a); \
-        else ens_march_kernel<R, MINB, false><<<grid, ENS_MARCH_THREADS, 0, e->stream>>>(a);    \
+        (ref ? mom ? ens_march_kernel<R, MINB, true, LB_PSI_REF>                               \
+                   : ens_march_kernel<R, MINB, false, LB_PSI_REF>                              \
+             : mom ? ens_march_kernel<R, MINB, true, LB_PSI_EXP1>                              \
+                   : ens_march_kernel<R, MINB, false, LB_PSI_EXP1>)                            \
+            <<<grid, ENS_MARCH_THREADS, 0, e->stream>>>(a);                                    \
         break;
             LB_ENS_MARCH(LB_ENS_MLAUNCH)
 #undef LB_ENS_MLAUNCH
@@ -660,7 +663,8 @@ cudaError_t ens_step(lb_ensemble *e, int from, bool mom) {
         return cudaGetLastError();
     }
     const dim3 block(e->shape.bx, e->shape.ry);
-    ens_density_kernel<<<grid, block, 0, e->stream>>>(a);
+    if (ref) ens_density_kernel<LB_PSI_REF><<<grid, block, 0, e->stream>>>(a);
+    else ens_density_kernel<LB_PSI_EXP1><<<grid, block, 0, e->stream>>>(a);
     cudaError_t c = cudaGetLastError();
     if (c != cudaSuccess) return c;
     if (mom) ens_fused_kernel<true><<<grid, block, 0, e->stream>>>(a);

@@ -301,14 +301,7 @@ __device__ __forceinline__ void pair_bgk(const PairConst &c, const PairD3 &d, fl
     pair(16, 17, a7, d.r7, pair_sub(c, ey, ez));
 }
 
-// the pseudo-potential of the configured form (LB_PSI_REF = 0: the
-// reference's 4 exp(-200/rho); LB_PSI_EXP1: 1 - exp(-rho)), a compile-time
-// choice so that each kernel carries the code of one form only
-template <int PSI>
-__device__ __forceinline__ float psi_of(float rho) {
-    return PSI == 0 ? psi_ref(rho) : psi_exp1(rho);
-}
-
+// the pseudo-potential of both nodes
 template <int PSI>
 __device__ __forceinline__ float2 psi_of(const PairConst &c, float2 rho) {
     return PSI == 0 ? make_float2(psi_ref(rho.x), psi_ref(rho.y)) : pair_psi_exp1(c, rho);
@@ -369,7 +362,7 @@ __global__ void __launch_bounds__((StageShape<S, TX>::THREADS), (StageShape<S, T
                 const int i = tid - TX, hx = i < SS::PY ? -1 : TX, hy = i % SS::PY - 1;
                 float gh[19];
                 pull_stage<S, TX>(st, hx, hy, gh);
-                ps[hy + 1][hx + 2] = psi_of<PSI>(StepArith<S>::rho(gh, a));
+                ps[hy + 1][hx + 2] = psi_form<PSI>(StepArith<S>::rho(gh, a));
             }
         }
         if (__syncthreads_or(!ok)) {
