@@ -64,7 +64,7 @@ template <int Q> struct Pop {
     float *f[Q];
 };
 template <int Q> struct CPop {
-    const float *__restrict__ f[Q];
+    const float *f[Q];
 };
 
 // cell flag bits used by the kernels (the low two are the public LB_CELL_*)
@@ -74,6 +74,9 @@ enum : uint8_t {
     CELL_NEAR_WALL = 0x04,   // fluid cell with at least one wall neighbour
     CELL_SOLID_BOUND = 0x08, // reference mode: wall cell surrounded by walls
 };
+__device__ __forceinline__ bool moving_wall(uint8_t fl) {
+    return (fl & (CELL_WALL | CELL_MOVING)) == (CELL_WALL | CELL_MOVING);
+}
 
 __device__ __forceinline__ int wrap_dec(int v, int n) { return v == 0 ? n - 1 : v - 1; }
 __device__ __forceinline__ int wrap_inc(int v, int n) { return v == n - 1 ? 0 : v + 1; }
@@ -81,8 +84,13 @@ __device__ __forceinline__ int wrap_add(int v, int c, int n) {
     return c > 0 ? wrap_inc(v, n) : (c < 0 ? wrap_dec(v, n) : v);
 }
 
-// streaming loads: read-only for the kernel's lifetime, touched once per step
-__device__ __forceinline__ float ld_stream(const float *p) { return __ldg(p); }
+// A value that an earlier launch wrote.  ld.global.nc is for data that are read-only
+// for the kernel's lifetime, and nothing holds it below a wait: a programmatic
+// dependent (DEP), whose life begins while its predecessor still writes, takes a
+// plain load, which after_predecessor() orders.
+template <bool DEP, typename T> __device__ __forceinline__ T ld_stream(const T *p) {
+    return DEP ? *p : __ldg(p);
+}
 
 // Population storage.  FP32 stores f_k itself.  The 16-bit forms store the
 // deviation d_k = f_k - wr_k from an offset wr_k = w_k * rho_ref (rounded to
@@ -97,7 +105,9 @@ template <> struct Store<float> {
     static constexpr int kind = 0;
     __device__ __forceinline__ static float load(const float *p, float) { return __ldg(p); }
     __device__ __forceinline__ static void store(float *p, float v, float) { *p = v; }
-    __device__ __forceinline__ static float load_dev(const float *p) { return __ldg(p); }
+    template <bool DEP> __device__ __forceinline__ static float load_dev(const float *p) {
+        return ld_stream<DEP>(p);
+    }
     __device__ __forceinline__ static void store_dev(float *p, float v) { *p = v; }
 };
 template <> struct Store<__half> {
@@ -108,8 +118,8 @@ template <> struct Store<__half> {
     __device__ __forceinline__ static void store(__half *p, float v, float wr) {
         *p = __float2half_rn(v - wr);
     }
-    __device__ __forceinline__ static float load_dev(const __half *p) {
-        return __half2float(__ldg(p));
+    template <bool DEP> __device__ __forceinline__ static float load_dev(const __half *p) {
+        return __half2float(ld_stream<DEP>(p));
     }
     __device__ __forceinline__ static void store_dev(__half *p, float d) {
         *p = __float2half_rn(d);
@@ -123,8 +133,8 @@ template <> struct Store<__nv_bfloat16> {
     __device__ __forceinline__ static void store(__nv_bfloat16 *p, float v, float wr) {
         *p = __float2bfloat16_rn(v - wr);
     }
-    __device__ __forceinline__ static float load_dev(const __nv_bfloat16 *p) {
-        return __bfloat162float(__ldg(p));
+    template <bool DEP> __device__ __forceinline__ static float load_dev(const __nv_bfloat16 *p) {
+        return __bfloat162float(ld_stream<DEP>(p));
     }
     __device__ __forceinline__ static void store_dev(__nv_bfloat16 *p, float d) {
         *p = __float2bfloat16_rn(d);

@@ -67,17 +67,22 @@ __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
 
     if (MODE == MODE_REF && (fl & CELL_WALL)) {
         const bool sb_self = a.sb[o] != 0;
+        float v[19];
 #pragma unroll
         for (int m = 0; m < 19; m++) {
-            float v;
             if (m == 0) {
-                v = ld_stream(a.src.f[0] + o);
+                v[m] = ld_stream<DEP>(a.src.f[0] + o);
             } else {
                 const int on = o + n.off(d3_cx(m), d3_cy(m), d3_cz(m));
                 const bool resp_sb = d3_pos(m) ? sb_self : (a.sb[on] != 0);
-                v = resp_sb ? ld_stream(a.src.f[m] + o) : ld_stream(a.src.f[d3_opp(m)] + on);
+                v[m] = resp_sb ? ld_stream<DEP>(a.src.f[m] + o)
+                               : ld_stream<DEP>(a.src.f[d3_opp(m)] + on);
             }
-            a.dst.f[m][o] = v;
+            if (!DEP) a.dst.f[m][o] = v[m];
+        }
+        if (DEP) {  // whose loads may not pass a store
+#pragma unroll
+            for (int m = 0; m < 19; m++) a.dst.f[m][o] = v[m];
         }
         if (MOM) { a.ux[o] = 0.f; a.uy[o] = 0.f; a.uz[o] = 0.f; a.rho[o] = 0.f; }
         if (PLOT) a.plot[o] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -92,11 +97,11 @@ __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
 
     float g[19];
     if (MODE == MODE_NATIVE) {
-        pull_native<S>(a, o, n, fl, g);
+        pull_native<S, false, DEP>(a, o, n, fl, g);
     } else {
 #pragma unroll
         for (int k = 0; k < 19; k++)
-            g[k] = ld_stream(a.src.f[k] + o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k)));
+            g[k] = ld_stream<DEP>(a.src.f[k] + o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k)));
         if (x == 0 && a.dev == 0)
             d3q19_zou_he_west(g, a.ux_in, a.inv_in);
         else if (x == a.W - 1 && a.dev == a.ndev - 1)
@@ -122,7 +127,7 @@ __global__ void __launch_bounds__(D3_BLOCK, (sizeof(S) == 2 && !SC) ? 12 : 0)
                 ps[0] = a.psi[o];
 #pragma unroll
                 for (int k = 1; k < 19; k++)
-                    ps[k] = __ldg(a.psi + o + n.off(d3_cx(k), d3_cy(k), d3_cz(k)));
+                    ps[k] = ld_stream<DEP>(a.psi + o + n.off(d3_cx(k), d3_cy(k), d3_cz(k)));
                 float IFx, IFy, IFz;
                 d3q19_sc_sum_native(ps, a.w1, a.w7, IFx, IFy, IFz);
                 const float c = (-a.G * ps[0]) * inv_rt;
@@ -156,7 +161,7 @@ __global__ void __launch_bounds__(D3_BLOCK) d3q19_density_kernel(const D3Args a)
     }
     const Nbr3 n(c.x, c.y, c.z, a.W, a.H, a.D);
     float g[19];
-    pull_native<S>(a, o, n, fl, g);
+    pull_native<S, false, DEP>(a, o, n, fl, g);
     const float rho = StepArith<S>::rho(g, a);
     a.psi[o] = psi_form<PSI>(rho);
 }

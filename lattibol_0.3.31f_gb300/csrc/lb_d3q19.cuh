@@ -41,30 +41,50 @@ struct Coord3 {
 // Native pull of the 19 populations of fluid node o (see d3q19_fused_kernel):
 // f_k in FP32 storage, the deviation d_k in 16-bit storage.  IDX32: each
 // upstream index is summed in 32 bits before the one pointer addition (fewer
-// instructions, a few more registers; for the issue-bound closure kernel).
-template <typename S, bool IDX32 = false>
+// instructions, a few more registers; for the issue-bound closure kernel).  DEP:
+// the kernel is a programmatic dependent (ld_stream); its loads near walls are not
+// hoisted over the tests of the upstream flags, so these all come first.
+template <typename S, bool IDX32 = false, bool DEP = false>
 __device__ __forceinline__ void pull_native(const D3Args &a, int o, const Nbr3 &n, uint8_t fl,
                                             float (&g)[19]) {
     const S *const *src = (const S *const *)(a.src.f);  // storage arrays behind float*
-    if (fl & CELL_NEAR_WALL) {
+    if (DEP && (fl & CELL_NEAR_WALL)) {
+        uint32_t wall = 0, moving = 0;  // bit k: the upstream node is a wall, a moving one
+#pragma unroll
+        for (int k = 1; k < 19; k++) {
+            const uint8_t fu = a.flags[o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k))];
+            wall |= (fu & CELL_WALL ? 1u : 0u) << k;
+            moving |= (moving_wall(fu) ? 1u : 0u) << k;
+        }
+#pragma unroll
+        for (int k = 0; k < 19; k++) {
+            const int up = o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k));
+            g[k] = Store<S>::template load_dev<DEP>(wall >> k & 1 ? src[d3_opp(k)] + o : src[k] + up);
+        }
+        if (moving) {
+#pragma unroll
+            for (int k = 1; k < 19; k++)
+                if (moving >> k & 1) g[k] = g[k] - a.corr[d3_opp(k)];
+        }
+    } else if (fl & CELL_NEAR_WALL) {
 #pragma unroll
         for (int k = 0; k < 19; k++) {
             const int up = o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k));
             const uint8_t fu = k == 0 ? 0 : a.flags[up];
             if (fu & CELL_WALL) {
-                const float v = Store<S>::load_dev(src[d3_opp(k)] + o);
+                const float v = Store<S>::template load_dev<DEP>(src[d3_opp(k)] + o);
                 g[k] = (fu & CELL_MOVING) ? v - a.corr[d3_opp(k)] : v;
             } else {
-                g[k] = Store<S>::load_dev(src[k] + up);
+                g[k] = Store<S>::template load_dev<DEP>(src[k] + up);
             }
         }
     } else {
 #pragma unroll
         for (int k = 0; k < 19; k++) {
             if (IDX32)
-                g[k] = Store<S>::load_dev(src[k] + (o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k))));
+                g[k] = Store<S>::template load_dev<DEP>(src[k] + (o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k))));
             else
-                g[k] = Store<S>::load_dev(src[k] + o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k)));
+                g[k] = Store<S>::template load_dev<DEP>(src[k] + o + n.off(-d3_cx(k), -d3_cy(k), -d3_cz(k)));
         }
     }
 }

@@ -137,7 +137,10 @@ __global__ void __launch_bounds__(32, MD_BLOCKS)
             if (WALLS) {
                 uint32_t *const m = reinterpret_cast<uint32_t *>(d - lane + 9 * 32) + lane;
                 if (ALIGNED) md_copy<4>(m, ma.mask + (o + xa));
-                else *m = (uint32_t)__ldg(ma.mask + (o + xa)) | (uint32_t)__ldg(ma.mask + (o + xb)) << 16;
+                else {
+                    const uint32_t lo = ld_stream<true>(ma.mask + (o + xa));
+                    *m = lo | (uint32_t)ld_stream<true>(ma.mask + (o + xb)) << 16;
+                }
             }
             y = wrap_inc(y, H);
         }

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(NT) d2q9_tblock_kernel(const D2Args a) {
         const int o = gx + W * gy;
         fl[i] = a.flags[o];
 #pragma unroll
-        for (int k = 0; k < 9; k++) b0[k * RN + i] = ld_stream(a.src.f[k] + o);
+        for (int k = 0; k < 9; k++) b0[k * RN + i] = ld_stream<true>(a.src.f[k] + o);
     }
     __syncthreads();
     TbSteps<RX, RY, NT, TS, 1>::run(a, b0, b1, fl, corr);
