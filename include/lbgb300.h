@@ -288,10 +288,11 @@ int lb_ensemble_get_moments(lb_ensemble *e, float *rho, float *ux, float *uy);
  * at 40; 5: 32 x 32 at 60), 6..9 warps marching down 32-column strips with
  * psi of three rows in registers (6: 32 rows at 80 registers; 7: 32 rows at
  * 64; 8: 64 rows; 9: 16 rows), 10..12 strips of column
- * pairs, two nodes per lane (10, the default: rows per strip of the library's
+ * pairs, two nodes per lane (10: rows per strip of the library's
  * choice, and two steps per launch on ensembles of 2^20 nodes and more whose
  * domains' rows mostly start on 16 bytes; 11: 64 rows; 12: 16 rows; blocks per
- * SM do not apply).  Otherwise the two-pass step (psi pass, fused pass)
+ * SM do not apply).  The default is 10, or 6 on ensembles of many domains of up
+ * to some 24 columns, where a strip of column pairs lies mostly idle.  Otherwise the two-pass step (psi pass, fused pass)
  * over groups of `rows` rows with threads_x threads along x (a multiple of
  * 32).  Both give the same bits.  The autotuner times every candidate for
  * trial_steps steps on the ensemble itself (advancing its state: tune before

@@ -569,8 +569,7 @@ struct lb_ensemble {
     bool two_steps = false;  // form 10 advances two steps per launch
     int pair_rows = 0;       // column-pair strips: rows of an item
     int cur = 0, psi_form = LB_PSI_EXP1, sms = 1, graph_steps = 32;
-    // strips of column pairs
-    LaunchShape shape{0, 10, 12};
+    LaunchShape shape{0, 10, 12};  // strips of column pairs (or form 6: ens_strips_pay)
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -716,6 +715,40 @@ int ens_pick_rows(const lb_ensemble *e) {
     return pick;
 }
 
+// Whether the strips of 32 columns (form 6) are the default: on many narrow domains
+// most of a 64-column strip lies idle, and rows that do not start on 16 bytes are
+// copied node by node.  us per step, column pairs / strips: 65 625 domains of 8^2 352 /
+// 249, 16 384 of 16^2 140 / 126, 42 000 of 10^2 393 / 194, 5 242 of 10^2 55 / 30, 12 962
+// of 18^2 157 / 114; but 512 of 16^2 9.5 / 15, 5 357 of 28^2 76 / 91, 1 310 of 20^2 both
+// 25.  The two times are estimated as an item's march times us per row (a warp's row
+// of pairs; dearer where it is copied by node) times a function of the rounds of items
+// w; over 98 ensembles of 2^2 .. 56^2 domains (4 000 .. 4.2 M nodes) the estimates'
+// choice lost at most 9 % to the other form, but for one of 24 %.
+struct EnsEstimate {
+    double items = 0, sum = 0;  // items; their marches in us
+    void add(int count, int rows, double us_per_row) {
+        items += count;
+        sum += count * (double)rows * us_per_row;
+    }
+};
+bool ens_strips_pay(const lb_ensemble *e) {
+    const int steps = e->two_steps ? 2 : 1, r = ens_pick_rows(e), R = ens_march_rows(6);
+    EnsEstimate pairs, strips;
+    for (const EnsDomain &m : e->dom) {
+        const int tw = ens_pair_tile(m.W), k = (m.H + r - 1) / r, n = (m.H + R - 1) / R;
+        const double row = ((m.W | m.off) & 3) == 0 ? (steps == 1 ? 1.2 : 1.5)
+                                                    : (1.1 + 8. / std::min(m.W, tw)) *
+                                                          (steps == 1 ? 1. : 1.25);
+        pairs.add((m.W + tw - 1) / tw * k, (m.H + k - 1) / k + 4 * steps, row);
+        strips.add((m.W + ET_BX - 1) / ET_BX * n, (m.H + n - 1) / n + 2, 1.7);
+    }
+    const double wp = pairs.items / ((double)e->sms * ep_blocks(steps));
+    const double ws = strips.items / (e->sms * 3. * (ENS_MARCH_THREADS / 32));
+    const double fp = wp <= 1. ? std::min(1., 0.2 + 1.1 * wp) : std::max(1.42, 0.32 + 0.82 * wp);
+    const double fs = ws <= 1. ? 0.5 + 0.5 * ws : 0.32 + 0.82 * ws;
+    return strips.sum / strips.items * fs < 0.95 * pairs.sum / pairs.items * fp / steps;
+}
+
 // work list of row groups for the current shape
 int build_items(lb_ensemble *e) {
     std::vector<EnsItem> items;
@@ -817,6 +850,7 @@ int lb_ensemble_create(int nd, const int *nx, const int *ny, const float *G, con
         lb_ensemble_destroy(e);
         return c == cudaErrorMemoryAllocation ? LB_ERR_NOMEM : LB_ERR_CUDA;
     }
+    if (ens_strips_pay(e)) e->shape = LaunchShape{0, 6, 6};
     if (build_items(e) != LB_OK) {
         lb_ensemble_destroy(e);
         return LB_ERR_CUDA;
