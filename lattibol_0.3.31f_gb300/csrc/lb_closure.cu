@@ -1082,8 +1082,8 @@ int lb_mlp_create(uint64_t seed, lb_mlp **out) {
     if (e == cudaSuccess) e = cudaMalloc(&m->w1b, sizeof(__nv_bfloat16) * MLP_H * MLP_IN_PAD);
     if (e == cudaSuccess) e = cudaMalloc(&m->w2b, sizeof(__nv_bfloat16) * 2 * MLP_H * MLP_H);
     if (e == cudaSuccess) e = cudaMalloc(&m->err_dev, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(m->err_dev, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->err_dev, 0, sizeof(int), m->stream);
     if (e != cudaSuccess) {
         lb_mlp_destroy(m);
         return LB_ERR_NOMEM;

@@ -248,7 +248,7 @@ int check_device_error(lb_ctx *c) {
            cudaMemcpy(&word, c->errw, sizeof(int), cudaMemcpyDeviceToHost));
     c->err_pending = false;
     if (word != 0) {
-        LB_TRY(c, "device error word", cudaMemset(c->errw, 0, sizeof(int)));
+        LB_TRY(c, "device error word", cudaMemsetAsync(c->errw, 0, sizeof(int), c->stream));
         return fail(c, LB_ERR_DEVICE,
                     "a kernel gave up waiting on the GPU (tensor-core MMA or staged copies)");
     }
@@ -519,8 +519,8 @@ int lb_create(const lb_config *cfg, lb_ctx **out) {
     if (e == cudaSuccess) e = cudaMalloc(&c->red, sizeof(double) * (reduce_partials_size() + 16));
     if (e == cudaSuccess)
         e = cudaMalloc(&c->errw, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->errw, 0, sizeof(int), c->stream);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->errw, 0, sizeof(int), c->stream);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->flags, 0, c->stride, c->stream);
@@ -1545,13 +1545,19 @@ int lb_malloc_host(void **p, size_t bytes) {
 }
 int lb_free_host(void *p) { return cudaFreeHost(p) == cudaSuccess ? LB_OK : LB_ERR_CUDA; }
 int lb_memcpy_h2d(void *dst, const void *src, size_t bytes) {
-    return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess ? LB_OK : LB_ERR_CUDA;
+    // complete for every stream (the contexts' do not wait for the legacy one): a copy
+    // from pageable memory may return before its last bytes have arrived
+    cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e == cudaSuccess ? LB_OK : LB_ERR_CUDA;
 }
 int lb_memcpy_d2h(void *dst, const void *src, size_t bytes) {
     return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost) == cudaSuccess ? LB_OK : LB_ERR_CUDA;
 }
 int lb_memset(void *dst, int value, size_t bytes) {
-    return cudaMemset(dst, value, bytes) == cudaSuccess ? LB_OK : LB_ERR_CUDA;
+    cudaError_t e = cudaMemset(dst, value, bytes);  // as above
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e == cudaSuccess ? LB_OK : LB_ERR_CUDA;
 }
 int lb_device_synchronize(void) {
     return cudaDeviceSynchronize() == cudaSuccess ? LB_OK : LB_ERR_CUDA;

@@ -780,8 +780,11 @@ int build_items(lb_ensemble *e) {
         LB_ETRY(e, "work list", cudaMalloc(&e->items_d, sizeof(EnsItem) * items.size()));
         e->items_cap = (int)items.size();
     }
-    LB_ETRY(e, "work list", cudaMemcpy(e->items_d, items.data(), sizeof(EnsItem) * items.size(),
-                                       cudaMemcpyHostToDevice));
+    // in the steps' stream: a plain copy from pageable memory may return before its
+    // last bytes have arrived, and a stream that does not block would not wait for them
+    LB_ETRY(e, "work list", cudaMemcpyAsync(e->items_d, items.data(), sizeof(EnsItem) * items.size(),
+                                            cudaMemcpyHostToDevice, e->stream));
+    LB_ETRY(e, "work list", cudaStreamSynchronize(e->stream));
     e->nitems = (int)items.size();
     drop_graphs(e);
     return LB_OK;
@@ -842,8 +845,8 @@ int lb_ensemble_create(int nd, const int *nx, const int *ny, const float *G, con
     if (c == cudaSuccess) c = cudaMalloc(&e->pop[1], sizeof(float) * 9 * e->stride);
     if (c == cudaSuccess) c = cudaMalloc(&e->psi, sizeof(float) * e->stride);
     if (c == cudaSuccess) c = cudaMalloc(&e->mom, sizeof(float) * 3 * e->stride);
-    if (c == cudaSuccess) c = cudaMemset(e->mom, 0, sizeof(float) * 3 * e->stride);
     if (c == cudaSuccess) c = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
+    if (c == cudaSuccess) c = cudaMemsetAsync(e->mom, 0, sizeof(float) * 3 * e->stride, e->stream);
     if (c == cudaSuccess) c = cudaEventCreate(&e->ev0);
     if (c == cudaSuccess) c = cudaEventCreate(&e->ev1);
     if (c != cudaSuccess) {
