@@ -292,8 +292,9 @@ int lb_ensemble_get_moments(lb_ensemble *e, float *rho, float *ux, float *uy);
  * choice, and two steps per launch on ensembles of 2^20 nodes and more whose
  * domains' rows mostly start on 16 bytes; 11: 64 rows; 12: 16 rows; blocks per
  * SM do not apply).  The default is 10, or 6 on ensembles of many domains of up
- * to some 24 columns, where a strip of column pairs lies mostly idle.  Otherwise the two-pass step (psi pass, fused pass)
- * over groups of `rows` rows with threads_x threads along x (a multiple of
+ * to some 24 columns, where a strip of column pairs lies mostly idle.
+ * Otherwise (threads_x > 0) the two-pass step (psi pass, fused pass) over
+ * groups of `rows` rows with threads_x threads along x (a multiple of
  * 32).  Both give the same bits.  The autotuner times every candidate for
  * trial_steps steps on the ensemble itself (advancing its state: tune before
  * initialising) and keeps the fastest, returned in out[3] */

@@ -480,13 +480,13 @@ __global__ void features_kernel(const float *fl, int Wc, int Hc, int Dc, float n
 // of a tile, row t of the sample-major MMA tiles, column t of the transposed
 // (sample-contracted) tiles and lane t of tensor memory; in training threads t
 // and t + 128 share them, each with half of the hidden columns (the launch is
-// one tile per block, a latency chain of five MMA groups and the epilogues
+// one tile per block, a latency chain of four waits for MMAs and the epilogues
 // between them: half as many columns per thread, and block sums stored in rows
 // of consecutive floats, took a step of 16 384 samples from 14.2 to 10.9 us;
 // 20.2 before the launches overlapped).  The output's sum over all 64 columns
-// is formed by both, in the one order.  Thread 0 issues every MMA (BF16 operands in shared memory, K-major core matrices,
-// lb_tc05.cuh; FP32 accumulators in tensor memory) and commits it to one
-// mbarrier.  Per tile:
+// is formed by both, in the one order.  Thread 0 issues every MMA (BF16 operands
+// in shared memory, K-major core matrices, lb_tc05.cuh; FP32 accumulators in
+// tensor memory) and commits it to one mbarrier.  Per tile:
 //   1. x (19 features, padded to 32) -> row t of A; D_h1 = A W1^T;
 //   2. h1 = ReLU(D_h1 + b1) as BF16 -> row t of A (K 64) and column t of
 //      H1^T; D_h2 = A W2^T;
@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(TRAIN ? 256 : 128, 1) mlp_tc_kernel(const MlpD
         if (!ok) break;
     }
     if (TRAIN && ok) {
-        // the block's sums in the order of NetSums: rows 0-63 of the accumulators
+        // the block's sums in the order of SUM_W2 .. SUM_LOSS: rows 0-63 of the accumulators
         // (t < 64) hold dW2, db2 and dw3, rows 64-127 dW1 and db1, row 64 db3;
         // the threads' halves take half of the columns each
         float *pb = out + (long)blockIdx.x * NGRAD;

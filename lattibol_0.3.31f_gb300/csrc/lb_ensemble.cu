@@ -3,16 +3,18 @@
 //
 // All domains live in one packed structure-of-arrays slab (domain d occupies
 // nodes [off_d, off_d + W_d*H_d), node x + W_d*y inside it), in two
-// population sets that alternate like the single-lattice context.  A step is
-// two persistent launches over a host-built work list of row groups (a
-// domain's extents and physics and a first row): the density pass writes psi = psi(rho) of every node,
-// the fused pass pulls the populations, adds the Shan-Chen shift from the
-// 3x3 psi stencil and relaxes.  Each block walks the work list with a stride
-// of the grid size, and the grid is a multiple of the SM count, so uneven
-// domain sizes do not leave SMs idle.  Batches of steps are replayed from a
-// captured CUDA graph.  The launch shape (threads along x, rows per item,
-// blocks per SM) is chosen by lb_ensemble_autotune, which times each
-// candidate on the ensemble itself.
+// population sets that alternate like the single-lattice context.  A step
+// walks a host-built work list (a domain's extents and physics, a first row
+// and column).  By default one launch advances one or two steps by strips of
+// column pairs, or by strips of 32 columns on ensembles of many narrow domains
+// (ens_strips_pay); the other forms are tiles, and two persistent launches
+// over row groups: the density pass writes psi = psi(rho) of every node, the
+// fused pass pulls the populations, adds the Shan-Chen shift from the 3x3 psi
+// stencil and relaxes.  In the persistent forms each block walks the list with
+// a stride of the grid size, and the grid is a multiple of the SM count, so
+// uneven domain sizes do not leave SMs idle.  Batches of steps are replayed
+// from a captured CUDA graph.  lb_ensemble_autotune times each form on the
+// ensemble itself.
 //
 // The per-node arithmetic is the single-domain native D2Q9 Shan-Chen step's
 // (same device functions, same order: d2q9_moments_native,
@@ -129,7 +131,7 @@ __global__ void ens_fused_kernel(const EnsArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Single-pass step over tiles of 32 x BY nodes (the default launch).  A
+// Single-pass step over tiles of 32 x BY nodes.  A
 // block pulls its tile nodes (one per thread) and the ring of nodes around
 // them (84 for 32 x 8 tiles), forms psi of all of them in shared memory, and then relaxes
 // its tile nodes with the Shan-Chen shift from the shared psi tile.  psi never
@@ -319,8 +321,8 @@ __global__ void __launch_bounds__(ENS_MARCH_THREADS, MINB) ens_march_kernel(cons
 // 64..128 31, 30 (9: one item per warp of an eight-warp block left most SMs
 // empty).  About 180 issue slots per 64 node updates, 347 per 32 for the row
 // ring.  Two steps move 40 B per node update and are bound by the latency of
-// their arithmetic chain at 12 warps per SM (168 registers), one step by
-// memory and the chain at 16.
+// their arithmetic chain at 12 warps per SM (168 registers, 56 bytes of them
+// spilled), one step by memory and the chain at 16 (128 registers).
 // ---------------------------------------------------------------------------
 constexpr int EP_EDGE = 4, EP_COLS = 64 - 2 * EP_EDGE;
 constexpr int EP_RING = 4;
@@ -552,10 +554,13 @@ int ens_pair_tile(int W) {
 
 }  // namespace
 
-// Form 10 takes two steps per launch from this many nodes on (24 domains of 0.27
-// M nodes in all: 31.5 GLUPS with two, 30.2 with one; 64 of 6.6 M: 88 and 77) if
-// most of them lie in domains whose rows start on 16 bytes (400 domains of 97,
-// 101 and 130 columns: 39 GLUPS with two, 52 with one).
+// Form 10 takes two steps per launch from this many nodes on if most of them lie in
+// domains whose rows start on 16 bytes (400 domains of 97, 101 and 130 columns: 39
+// GLUPS with two, 52 with one).  Time of two over one on such ensembles: 512 domains
+// of 32..512 0.80, 64 of them 0.86, 255 of 64^2 (1.04 M nodes) 1.00; below the line it
+// depends on how the items fill the warps: 60 of 128^2 0.92, 10 of 256^2 (0.66 M) 0.79,
+// 128 of 64^2 0.99, but 6 of 256^2 (0.39 M) 1.21, 64 of 64^2 1.20, 2048 of 16^2 1.17, 16
+// of 128^2 0.97; over 37 ensembles of up to 0.98 M nodes 0.78 .. 1.21.
 constexpr long ENS_TWO_STEP_MIN_NODES = 1L << 20;
 
 struct lb_ensemble {
@@ -997,9 +1002,9 @@ int lb_ensemble_get_launch(const lb_ensemble *e, int out[3]) {
 }
 
 // Times every candidate shape for trial_steps steps (after one untimed step)
-// on the ensemble's current state and keeps the fastest.  The state advances
-// by (trial_steps + 1) steps per candidate: tune before setting the initial
-// state.
+// on the ensemble's current state and keeps the fastest.  The state advances by
+// (trial_steps + 1) steps per candidate, by up to two more where a launch is two
+// steps: tune before setting the initial state.
 int lb_ensemble_autotune(lb_ensemble *e, int trial_steps, int out[3]) {
     if (!e || trial_steps < 1) return LB_ERR_ARG;
     // the single-pass tiles, then the two-pass row groups {64, 128, 256

@@ -130,13 +130,19 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
 }
 
 // One of a step's kernels, one thread per node: a dependent launch where the
-// start of a launch weighs, on grids of up to 2432 blocks (16 per SM, one wave),
-// and on the legacy default stream, which runs beside no other.  Three lattices
-// side by side, GLUPS without and with: 45 x 23 x 17 7.4, 10.5; 100 x 45 x 40 49, 61;
-// 16 x 13 x 187 (2431 blocks) 14.2, 15.6; beyond, 64^3 46, 53, but 30 x 64 x 64 36, 29
-// and 120 x 40 x 100 46.9, 46.3: on grids of short blocks after_predecessor itself
-// costs (30 x 157 x 126 in FP16, 19 782 blocks: 26, 16), so `plain` is the kernel
+// start of a launch weighs.
+// A context's own stream: on grids of up to 2432 blocks (16 per SM of 152, one wave).
+// Three lattices side by side, GLUPS without and with: 45 x 23 x 17 7.4, 10.5; 100 x 45
+// x 40 49, 61; 16 x 13 x 187 (2431 blocks) 14.2, 15.6; beyond, 64^3 46, 53, but 30 x 64 x
+// 64 36, 29 and 120 x 40 x 100 46.9, 46.3: on grids of short blocks after_predecessor
+// itself costs (30 x 157 x 126 in FP16, 19 782 blocks: 26, 16), so `plain` is the kernel
 // without it.
+// The legacy default stream, which the entry points' loops fill from the host: always,
+// and so are the entry points' streaming and collision launches.  us per 20 steps of
+// such a loop, plain beyond 2432 blocks and always dependent: fused 64^3 412, 276, 30 x
+// 157 x 126 807, 651, 256 x 128 x 128 2665, 2415; streaming and collision apart, 64^3
+// 666, 598, 200 x 16 x 200 1062, 920, 20 x 5000 1080, 951, 256 x 128 x 128 7035, 6919
+// (slower on none of 46 shapes).
 template <typename Args>
 cudaError_t launch_step(void (*dependent)(Args), void (*plain)(Args), dim3 grid, dim3 block,
                         cudaStream_t s, const Args &a) {

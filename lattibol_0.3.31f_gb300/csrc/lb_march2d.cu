@@ -305,8 +305,8 @@ int march_steps_per_launch() { return T; }
 // rows that an item reads beyond its own.  A pass takes an item's march times a
 // function of the rounds of items w (a partly filled round runs its warps
 // faster, a nearly empty second one costs almost as much as a full one;
-// measured at 1568 x 1024, us per step: 16 rows, 1792 items for 1824 warps, 12.0;
-// 12 rows 14.8, 24 rows 14.1, 32 rows 16.8).
+// measured at 1568 x 1024, us per step: 16 rows, 1792 items for 1824 warps, 10.2;
+// 8 rows 12.6, 12 rows 12.7, 24 rows 13.5, 32 rows 12.8, 48 rows 16.9).
 MarchPlan march_plan(int W, int H) {
     MarchPlan p{};
     const int ns = (W + MD_COLS - 1) / MD_COLS;

@@ -38,7 +38,7 @@ __device__ __forceinline__ float2 pair_addp(const PairConst &c, float2 a, float2
 // single fused roundings, which Markstein's theorem (Markstein, "Computation
 // of elementary functions on the IBM RISC System/6000 processor", 1990) makes
 // the correctly rounded reciprocal.  The same bits as 1.f / x on all 2^32
-// arguments (compared one by one); where the residual says that the
+// arguments (tests/test_gpu_every_float.py); where the residual says that the
 // approximation is none (zero, infinite, NaN or subnormal x or 1 / x) the
 // divisions themselves run.  9 issue slots for the two lanes, against about 45
 // for two divisions and the moves around them.

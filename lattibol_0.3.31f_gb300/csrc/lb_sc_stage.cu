@@ -31,17 +31,19 @@
 // the paired FP32 instructions (lb_pairs.cuh), so the result is bit-identical
 // to the density pass + fused step.
 //
-// Measured at 256^3 (GLUPS FP32 / FP16 / BF16): 35.9 / 53.9 / 54.1; one node per
+// Measured at 256^3 (GLUPS FP32 / FP16 / BF16): 36.1 / 54.5 / 56.2; one node per
 // thread, 19 TMA boxes per stage for the interior tiles of 16-bit storage and
-// chunks of a divisor of the depth: 35.0 / 42.0 / 42.0; at 128^3 31.9 / 44.1
-// against 25.8 / 29.1, at 64^3 17.9 / 25.0 against 17.9 / 20.1.  (800 issue slots
+// chunks of a divisor of the depth: 35.0 / 42.0 / 42.0; at 128^3 31.8 / 45.3
+// against 25.8 / 29.1, at 64^3 19.6 / 27.2 against 17.9 / 20.1.  (800 issue slots
 // per node bound the 16-bit step then; now 375.)  With two nodes per thread the TMA
 // boxes (ten rows of 160 bytes, 48.5) lose to the cp.async chunks, which read
 // fewer bytes on the sides.  What bounds the step now: FP32, memory (the same
 // copies and stores without any arithmetic between them: 39); 16-bit, the
 // latency of a plane's chain (copies landed, pulls, psi, barrier, stencil,
 // relaxation) at 16 warps per SM, which their registers allow (the copies and
-// stores alone: 77).  Tried without gain: 3 stages ahead (54.6), populations
+// stores alone: 77); at that bound, 128, the compiler spills 28 to 48 bytes per
+// thread (80 to 188 bytes of loads), in FP32 (159 to 163 registers) none.  Tried
+// without gain (54.8 in the same runs): 3 stages ahead (54.6), populations
 // kept as 16-bit words (52.9; 37 at 24 warps per SM, whose 80 registers spill),
 // momentum formed when pulled (53.3), the barrier split into arrival and wait
 // around the moments (54.6), planes and chunks backwards on odd steps (54.7),
@@ -468,7 +470,9 @@ __global__ void __launch_bounds__((StageShape<S, TX>::THREADS), (StageShape<S, T
         for (int s = 0; s < SS::SLOTS; s++) mbar_inval(&full[s]);
 }
 
-// lattices that the staged kernel takes
+// Lattices that the staged kernel takes: whole tiles.  The chunks have not needed a
+// depth that is a multiple of 4 since chunk_planes takes any length; other depths are
+// untried here and take the two-pass step.
 bool sc_stage_fits(int W, int H, int D) { return W % 32 == 0 && H % ST_TY == 0 && D % 4 == 0; }
 
 namespace {
@@ -485,8 +489,8 @@ template <typename S> PairD3 pair_d3(const D3Args &a) {
 
 // Planes of a chunk: the fewest plane steps, a chunk's planes and the two beyond
 // its ends times the waves of blocks; a single wave that leaves SMs part empty
-// runs its blocks somewhat faster.  256^3 in FP16: 37 planes, 2.95 waves, 54.8
-// GLUPS; 32 planes (3.4 waves) 53.4, 16 planes 51.1, 64 planes 48.2.
+// runs its blocks somewhat faster.  256^3 in FP16: 37 planes, 2.95 waves, 54.5
+// GLUPS; 32 planes (3.4 waves) 53.0, 16 planes 51.4, 64 planes 47.4.
 int chunk_planes(long tiles, int D, int resident) {
     int pick = 1;
     double best = 0;
@@ -518,7 +522,7 @@ cudaError_t stage_launch(const D3Args &a, cudaStream_t s) {
                                  a, zc, ST_WAIT, pair_constants(), pair_d3<S>(a));
 }
 
-// 16-bit storage takes the wide tile where the width allows it (256^3: 53.9
+// 16-bit storage takes the wide tile where the width allows it (256^3: 54.5
 // GLUPS, the narrow one 51); in FP32 two stages of it leave room for one block
 // per SM (34.0, three blocks of the narrow tile 36.0).
 template <typename S, bool MOM, int PSI>
