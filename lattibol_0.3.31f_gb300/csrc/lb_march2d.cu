@@ -335,8 +335,13 @@ MarchPlan march_plan(int W, int H) {
 }
 
 // Whether the strips beat one launch per step (beyond 2^19 nodes).  From 32 rows on
-// they did on every shape measured (1.02 to 2.5 times; 135 shapes of 0.53 .. 2.7 M
-// nodes, with rows that start on 4, 8 and 16 bytes).  On fewer rows the 2 T rows that
+// they did on every shape without force or walls (1.02 to 2.5 times; 135 shapes of 0.53
+// .. 2.7 M nodes, with rows that start on 4, 8 and 16 bytes).  With a force, 96 shapes,
+// time over one launch per step's, one lattice alone: 0.43 .. 1.07 without walls, 0.40 ..
+// 1.01 with 5 % of them, 0.55 .. 1.20 in a box, above 1 only under 1.2 M nodes (a strip
+// along a wall marches longer, and one lattice is one round of them); three lattices
+// side by side, 21 shapes of 0.53 .. 1.2 M nodes: 0.55 .. 0.90, 0.46 .. 0.82 and 0.59 ..
+// 1.00 (925 x 622; with a disc between two walls 1.04).  On fewer rows the 2 T rows that
 // an item reads beyond its own can outweigh it: us per step, strips / one launch per
 // step, 700 001 x 1 17.6 / 6.4, 175 000 x 4 7.8 / 6.6, 53 125 x 16 9.9 / 8.2, but
 // 50 001 x 20 7.5 / 9.7 and 525 000 x 4 19.5 / 25.4.  There the plan's time is compared
